@@ -37,6 +37,7 @@
 
 #include "hhs_ctx.h"
 #include "hhs_kernels.h"
+#include "hhs_kick64.cuh"
 #include "hhs_pairmath.cuh"
 #include "hhs_scan.cuh"
 #include "hhs_tma.cuh"
@@ -52,6 +53,7 @@ constexpr int kTX = 256;          // slow records per tile of the symmetric grid
 constexpr int kTW = 256;          // widest column tile of the packed grid timestep
 constexpr int kMaxFsb = 64;       // fast super-blocks of that kick (column-partial slots)
 constexpr int kMaxChunks = 32;    // source chunks per node (partial-sum slots)
+constexpr int kK64Pairs = 2048;   // pair terms per stage of the FP64 kick
 constexpr int kMaxLevels = 64;    // per-level state is kept in 64-bit masks
 constexpr unsigned long long kBarrierTimeoutNs = 60ull * 1000000000ull;
 
@@ -191,7 +193,7 @@ struct __align__(16) Smem {
             float colred[2][kEB / 32][kTW];
         } ts2;
         struct { float4 P0[kEB], P1[kEB], P2[kEB]; float2 M[kEB]; } kx;  // packed kick tiles
-        struct { double x[kEB], y[kEB], z[kEB], m[kEB]; } kd;   // FP64 kick tiles
+        Kick64Smem<kK64Pairs> k64;                              // FP64 kick terms
         struct {                                                  // tiny-subtree state
             double x[32], y[32], z[32], vx[32], vy[32], vz[32], m[32], ts[32];
             float4 A[32], B[32], V[32];
@@ -786,11 +788,100 @@ __device__ void ts_sym_tiles(const EParams& E, int n, int cw, long long u0, long
     __syncthreads();
 }
 
+// ---------------------------------------------------------------- FP64 kick units
+// The FP64 launch keeps (x, y, z, mass) of a level's slow particles in the same array (32
+// bytes a record, as the pairs of the mixed one).
+__device__ __forceinline__ double4* pk64_level(const EParams& E, int lvl) {
+    return reinterpret_cast<double4*>(E.pk + (size_t)lvl * (size_t)E.pk_stride * 4);
+}
+// Sinks s in [0, nf + ns): s < nf -> F[s] (fast), else L[s - nf] (slow). Slow sources are
+// drifted by h on the fly; fast sinks see slow sources only. A unit is a block of T sinks
+// of one kind; its sums go to k_part (slow sources in slots 0-2, fast sources in 3-5).
+__device__ void kick_fp64_block(const EParams& E, const int32_t* F, const int32_t* L, int nf,
+                                int ns, double h, const double4* PK, int s0, int s1, int cs,
+                                Smem& sm) {
+    const SoA& P = E.P;
+    auto& K = sm.u.k64;
+    const bool slow = s0 >= nf;
+    const int tid = threadIdx.x, T = kK64Pairs >> cs, nsink = s1 - s0;
+    // a slow particle at its kick position: its packed record, or drifted here
+    auto drifted = [&](int q, double& x, double& y, double& z, double& m) {
+        if (PK) {
+            const double2* r = reinterpret_cast<const double2*>(PK + q);
+            const double2 a = r[0], b = r[1];
+            x = a.x; y = a.y; z = b.x; m = b.y;
+        } else {
+            x = f64_add(P.x[q], f64_mul(P.vx[q], h));
+            y = f64_add(P.y[q], f64_mul(P.vy[q], h));
+            z = f64_add(P.z[q], f64_mul(P.vz[q], h));
+            m = P.m[q];
+        }
+    };
+    if (tid < nsink) {
+        double x, y, z, m;
+        if (slow) {
+            drifted(PK ? s0 - nf + tid : L[s0 - nf + tid], x, y, z, m);
+        } else {
+            const int g = F[s0 + tid];
+            x = P.x[g]; y = P.y[g]; z = P.z[g];
+        }
+        K.sx[tid] = x; K.sy[tid] = y; K.sz[tid] = z;
+    }
+    __syncthreads();
+    const int c = tid / T, s = tid & (T - 1);
+    const bool out = c < 3 && s < nsink;
+    // one loop for both kinds of sources: a single copy of the inlined pair code
+    for (int p = 0; p < (slow && nf > 0 ? 2 : 1); p++) {
+        const int32_t* S = p ? F : (PK ? nullptr : L);
+        const double a = kick64_sums(K, cs, nsink, p ? nf : ns, E.eps2,
+                                     [&](int j) { return list_at(S, j); },
+                                     [&](int g, double& x, double& y, double& z, double& m) {
+                                         if (p) {
+                                             x = P.x[g]; y = P.y[g]; z = P.z[g]; m = P.m[g];
+                                         } else {
+                                             drifted(g, x, y, z, m);
+                                         }
+                                     });
+        if (out) E.k_part[(size_t)(3 * p + c) * E.n_max + s0 + s] = a;
+    }
+}
+
+// Sinks [lo, hi) of the node over the workers: the slow blocks first (they see every
+// source), then the fast ones. Blocks of 8 sinks while those give the workers at most
+// kK64Rounds blocks each (the finest split; a stage's additions are then 256 long), else of
+// 32 (64 long): at N=16384 the kicks take 30.9 ms with one round, 23.8 with two or eight. PK: the slow particles packed at their kick positions (null: gathered from the
+// state arrays and drifted here). ctr: a work counter (null: blocks are dealt round robin).
+constexpr int kK64Rounds = 4;
+__device__ void kick_fp64_units(const EParams& E, const int32_t* F, const int32_t* L, int nf,
+                                int ns, double h, const double4* PK, int lo, int hi,
+                                unsigned* ctr, const Workers& W, Smem& sm) {
+    const int f0 = min(lo, nf), f1 = min(hi, nf), l0 = max(lo, nf), l1 = max(hi, nf);
+    auto shift = [&](int cnt) { return cnt <= 8 * kK64Rounds * W.count ? 8 : 6; };
+    const int csf = shift(f1 - f0), css = shift(l1 - l0);
+    const int Tf = kK64Pairs >> csf, Ts = kK64Pairs >> css;
+    const int us = (l1 - l0 + Ts - 1) / Ts, units = us + (f1 - f0 + Tf - 1) / Tf;
+    int u = W.id;
+    if (ctr) {
+        if (threadIdx.x == 0) sm.bcast = (int)atomicAdd(ctr, 1u);
+        __syncthreads();
+        u = sm.bcast;
+    }
+    while (u < units) {
+        __syncthreads();  // every thread has read sm.bcast
+        if (ctr && threadIdx.x == 0) sm.bcast = (int)atomicAdd(ctr, 1u);
+        const bool slow = u < us;
+        const int s0 = slow ? l0 + u * Ts : f0 + (u - us) * Tf;
+        kick_fp64_block(E, F, L, nf, ns, h, PK, s0, min(slow ? l1 : f1, s0 + (slow ? Ts : Tf)),
+                        slow ? css : csf, sm);
+        u = ctr ? sm.bcast : u + W.count;
+    }
+    __syncthreads();
+}
+
 // ---------------------------------------------------------------- kick units
-// Sinks s in [0, nf + ns): s < nf -> F[s] (fast), else L[s - nf] (slow). Sources j in
-// [0, ns + nf): j < ns -> L[j] (drifted by h on the fly), else F[j - ns]. Fast sinks
-// see slow sources only.
-template <int PREC>
+// Mixed kick of one block of kEB sinks from the sources [j0, j1): sinks s in [0, nf + ns) as
+// above; sources j < ns -> L[j] (drifted by h on the fly), else F[j - ns]. Fast sinks see
+// slow sources only.
 __device__ void kick_unit(const EParams& E, const int32_t* F, const int32_t* L, int nf, int ns,
                           double h, int ib, int jc, int j0, int j1, Smem& sm) {
     const int n = nf + ns;
@@ -801,114 +892,66 @@ __device__ void kick_unit(const EParams& E, const int32_t* F, const int32_t* L, 
     const int jend = slow ? j1 : min(j1, ns);
     const SoA& P = E.P;
     const int n_max = E.n_max;
-    if (PREC == HHS_PREC_FP64) {
-        double xi = 0, yi = 0, zi = 0;
+    DS xi{0, 0}, yi{0, 0}, zi{0, 0};
+    if (act) {
+        double x = P.x[g], y = P.y[g], z = P.z[g];
+        if (slow) { x = fma(P.vx[g], h, x); y = fma(P.vy[g], h, y); z = fma(P.vz[g], h, z); }
+        xi = ds_split(x); yi = ds_split(y); zi = ds_split(z);
+    }
+    float acc[3] = {0, 0, 0}, cmp[3] = {0, 0, 0};
+    for (int t0 = j0; t0 < j1; t0 += kEB) {
+        const int tl = min(kEB, j1 - t0);
+        __syncthreads();
+        if ((int)threadIdx.x < tl) {
+            const int j = t0 + threadIdx.x;
+            const bool js = j < ns;
+            const int gj = js ? L[j] : F[j - ns];
+            double x = P.x[gj], y = P.y[gj], z = P.z[gj];
+            if (js) { x = fma(P.vx[gj], h, x); y = fma(P.vy[gj], h, y); z = fma(P.vz[gj], h, z); }
+            const DS a = ds_split(x), b = ds_split(y), c = ds_split(z);
+            sm.u.km.A[threadIdx.x] = make_float4(a.hi, b.hi, c.hi, (float)P.m[gj]);
+            sm.u.km.B[threadIdx.x] = make_float4(a.lo, b.lo, c.lo, 0.0f);
+        }
+        __syncthreads();
         if (act) {
-            xi = P.x[g]; yi = P.y[g]; zi = P.z[g];
-            if (slow) {
-                xi = f64_add(xi, f64_mul(P.vx[g], h));
-                yi = f64_add(yi, f64_mul(P.vy[g], h));
-                zi = f64_add(zi, f64_mul(P.vz[g], h));
-            }
-        }
-        double aL[3] = {0, 0, 0}, aF[3] = {0, 0, 0};
-        for (int t0 = j0; t0 < j1; t0 += kEB) {
-            const int tl = min(kEB, j1 - t0);
-            __syncthreads();
-            if ((int)threadIdx.x < tl) {
-                const int j = t0 + threadIdx.x;
-                const bool js = j < ns;
-                const int gj = js ? L[j] : F[j - ns];
-                double x = P.x[gj], y = P.y[gj], z = P.z[gj];
-                if (js) {
-                    x = f64_add(x, f64_mul(P.vx[gj], h));
-                    y = f64_add(y, f64_mul(P.vy[gj], h));
-                    z = f64_add(z, f64_mul(P.vz[gj], h));
-                }
-                sm.u.kd.x[threadIdx.x] = x; sm.u.kd.y[threadIdx.x] = y;
-                sm.u.kd.z[threadIdx.x] = z; sm.u.kd.m[threadIdx.x] = P.m[gj];
-            }
-            __syncthreads();
-            if (act) {
-                const int je = min(tl, jend - t0);
-                for (int jl = 0; jl < je; jl++) {
-                    double* a = (t0 + jl < ns) ? aL : aF;
-                    kick_pair_fp64(f64_sub(sm.u.kd.x[jl], xi), f64_sub(sm.u.kd.y[jl], yi),
-                                   f64_sub(sm.u.kd.z[jl], zi), sm.u.kd.m[jl], a[0], a[1], a[2],
-                                   E.eps2);
-                }
-            }
-        }
-        if (act) {
-            double* part = E.k_part;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                part[(size_t)k * n_max + s] = aL[k];
-                part[(size_t)(3 + k) * n_max + s] = aF[k];
-            }
-        }
-    } else {
-        DS xi{0, 0}, yi{0, 0}, zi{0, 0};
-        if (act) {
-            double x = P.x[g], y = P.y[g], z = P.z[g];
-            if (slow) { x = fma(P.vx[g], h, x); y = fma(P.vy[g], h, y); z = fma(P.vz[g], h, z); }
-            xi = ds_split(x); yi = ds_split(y); zi = ds_split(z);
-        }
-        float acc[3] = {0, 0, 0}, cmp[3] = {0, 0, 0};
-        for (int t0 = j0; t0 < j1; t0 += kEB) {
-            const int tl = min(kEB, j1 - t0);
-            __syncthreads();
-            if ((int)threadIdx.x < tl) {
-                const int j = t0 + threadIdx.x;
-                const bool js = j < ns;
-                const int gj = js ? L[j] : F[j - ns];
-                double x = P.x[gj], y = P.y[gj], z = P.z[gj];
-                if (js) { x = fma(P.vx[gj], h, x); y = fma(P.vy[gj], h, y); z = fma(P.vz[gj], h, z); }
-                const DS a = ds_split(x), b = ds_split(y), c = ds_split(z);
-                sm.u.km.A[threadIdx.x] = make_float4(a.hi, b.hi, c.hi, (float)P.m[gj]);
-                sm.u.km.B[threadIdx.x] = make_float4(a.lo, b.lo, c.lo, 0.0f);
-            }
-            __syncthreads();
-            if (act) {
-                const int je = min(tl, jend - t0);
-                // blocked compensated summation: 32-pair FP32 blocks, Kahan across blocks
-                // (full blocks unrolled so that consecutive pairs overlap); 1/r^3 from
-                // rsqrtf with one Newton correction
-                auto pair = [&](int jl, float& bx, float& by, float& bz) {
-                    const float4 A = sm.u.km.A[jl], B = sm.u.km.B[jl];
-                    const float dx = ds_diff(A.x, B.x, xi.hi, xi.lo);
-                    const float dy = ds_diff(A.y, B.y, yi.hi, yi.lo);
-                    const float dz = ds_diff(A.z, B.z, zi.hi, zi.lo);
-                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, E.eps2f)));
-                    const float mr3 = mr3_nr(A.w, d2);
-                    bx = fmaf(dx, mr3, bx);
-                    by = fmaf(dy, mr3, by);
-                    bz = fmaf(dz, mr3, bz);
-                };
-                int jb = 0;
-                for (; jb + 32 <= je; jb += 32) {
-                    float bx = 0.0f, by = 0.0f, bz = 0.0f;
+            const int je = min(tl, jend - t0);
+            // blocked compensated summation: 32-pair FP32 blocks, Kahan across blocks
+            // (full blocks unrolled so that consecutive pairs overlap); 1/r^3 from
+            // rsqrtf with one Newton correction
+            auto pair = [&](int jl, float& bx, float& by, float& bz) {
+                const float4 A = sm.u.km.A[jl], B = sm.u.km.B[jl];
+                const float dx = ds_diff(A.x, B.x, xi.hi, xi.lo);
+                const float dy = ds_diff(A.y, B.y, yi.hi, yi.lo);
+                const float dz = ds_diff(A.z, B.z, zi.hi, zi.lo);
+                const float d2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, E.eps2f)));
+                const float mr3 = mr3_nr(A.w, d2);
+                bx = fmaf(dx, mr3, bx);
+                by = fmaf(dy, mr3, by);
+                bz = fmaf(dz, mr3, bz);
+            };
+            int jb = 0;
+            for (; jb + 32 <= je; jb += 32) {
+                float bx = 0.0f, by = 0.0f, bz = 0.0f;
 #pragma unroll 8
-                    for (int jl = jb; jl < jb + 32; jl++) pair(jl, bx, by, bz);
-                    kahan_add(acc[0], cmp[0], bx);
-                    kahan_add(acc[1], cmp[1], by);
-                    kahan_add(acc[2], cmp[2], bz);
-                }
-                if (jb < je) {
-                    float bx = 0.0f, by = 0.0f, bz = 0.0f;
-                    for (int jl = jb; jl < je; jl++) pair(jl, bx, by, bz);
-                    kahan_add(acc[0], cmp[0], bx);
-                    kahan_add(acc[1], cmp[1], by);
-                    kahan_add(acc[2], cmp[2], bz);
-                }
+                for (int jl = jb; jl < jb + 32; jl++) pair(jl, bx, by, bz);
+                kahan_add(acc[0], cmp[0], bx);
+                kahan_add(acc[1], cmp[1], by);
+                kahan_add(acc[2], cmp[2], bz);
+            }
+            if (jb < je) {
+                float bx = 0.0f, by = 0.0f, bz = 0.0f;
+                for (int jl = jb; jl < je; jl++) pair(jl, bx, by, bz);
+                kahan_add(acc[0], cmp[0], bx);
+                kahan_add(acc[1], cmp[1], by);
+                kahan_add(acc[2], cmp[2], bz);
             }
         }
-        if (act) {
-            double* part = E.k_part;
+    }
+    if (act) {
+        double* part = E.k_part;
 #pragma unroll
-            for (int k = 0; k < 3; k++)
-                part[(size_t)(jc * 3 + k) * n_max + s] = (double)acc[k] - (double)cmp[k];
-        }
+        for (int k = 0; k < 3; k++)
+            part[(size_t)(jc * 3 + k) * n_max + s] = (double)acc[k] - (double)cmp[k];
     }
 }
 
@@ -1882,13 +1925,20 @@ __device__ void split_phase(const EParams& E, const int32_t* S, int n, double dt
                 L[i - p] = gi;
                 q = i - p;
             }
-            if (PREC != HHS_PREC_FP64 && q >= 0 && E.pk && level < E.pk_levels) {
+            if (q >= 0 && E.pk && level < E.pk_levels) {
                 // packed kick source: the slow particle at its drifted kick position
                 const double h = dt * 0.5;
-                const DS x = ds_split(fma(E.P.vx[gi], h, E.P.x[gi]));
-                const DS y = ds_split(fma(E.P.vy[gi], h, E.P.y[gi]));
-                const DS z = ds_split(fma(E.P.vz[gi], h, E.P.z[gi]));
-                pk_put(pk_level(E, level), q, x, y, z, (float)E.P.m[gi]);
+                if constexpr (PREC == HHS_PREC_FP64) {
+                    double2* r = reinterpret_cast<double2*>(pk64_level(E, level) + q);
+                    r[0] = make_double2(f64_add(E.P.x[gi], f64_mul(E.P.vx[gi], h)),
+                                        f64_add(E.P.y[gi], f64_mul(E.P.vy[gi], h)));
+                    r[1] = make_double2(f64_add(E.P.z[gi], f64_mul(E.P.vz[gi], h)), E.P.m[gi]);
+                } else {
+                    const DS x = ds_split(fma(E.P.vx[gi], h, E.P.x[gi]));
+                    const DS y = ds_split(fma(E.P.vy[gi], h, E.P.y[gi]));
+                    const DS z = ds_split(fma(E.P.vz[gi], h, E.P.z[gi]));
+                    pk_put(pk_level(E, level), q, x, y, z, (float)E.P.m[gi]);
+                }
             }
         }
         if (t == ntiles - 1 && threadIdx.x == 0) {
@@ -3252,18 +3302,25 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     kp = kick_plan(nf, ns, W.count);
                     kick_sym_units(E, F, nf, ns, lvl, kp, 0, overlapped ? 2 : 0, sm);
                 }
-                for (int u = W.id; u < units; u += W.count) {
-                    int ib, jc;
-                    if (u < uf) {
-                        ib = u / jcs;
-                        jc = u % jcs;
-                    } else {
-                        ib = nfb + (u - uf) / nch;
-                        jc = (u - uf) % nch;
+                if constexpr (PREC == HHS_PREC_FP64) {
+                    unsigned* ctr = MODE == kModeGrid ? &E.st->kick_ctr[0][lvl] : nullptr;
+                    const double4* PK = MODE == kModeGrid && E.pk && lvl < E.pk_levels
+                                            ? pk64_level(E, lvl) : nullptr;
+                    kick_fp64_units(E, F, L, nf, ns, h, PK, 0, ntot, ctr, W, sm);
+                } else {
+                    for (int u = W.id; u < units; u += W.count) {
+                        int ib, jc;
+                        if (u < uf) {
+                            ib = u / jcs;
+                            jc = u % jcs;
+                        } else {
+                            ib = nfb + (u - uf) / nch;
+                            jc = (u - uf) % nch;
+                        }
+                        const int j0 = jc * C, j1 = min(ntot, j0 + C);
+                        if (x2) kick_unit_x2(E, F, L, nf, ns, h, ib, jc, j0, j1, sm);
+                        else kick_unit(E, F, L, nf, ns, h, ib, jc, j0, j1, sm);
                     }
-                    const int j0 = jc * C, j1 = min(ntot, j0 + C);
-                    if (x2) kick_unit_x2(E, F, L, nf, ns, h, ib, jc, j0, j1, sm);
-                    else kick_unit<PREC>(E, F, L, nf, ns, h, ib, jc, j0, j1, sm);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 const double ns_d = ns, nf_d = nf;
@@ -3487,15 +3544,15 @@ __global__ void __launch_bounds__(kEB, 2)
     kick_units_grid(E, F, nf, ns, lvl, nch, C, W, sm, ib_lo, ib_hi);
 }
 
-// FP64 kick units of sink blocks [ib_lo, ib_hi) (kEB sinks each), one chunk: slow then
-// fast sources in list order, the reference's order.
+// FP64 kick of the sinks [s_lo, s_hi): slow then fast sources in list order, the reference's
+// order.
 __global__ void __launch_bounds__(kEB, 2)
-    k_shard_kick_fp64(EParams E, const int32_t* F, const int32_t* L, int nf, int ns, int ib_lo,
-                      int ib_hi) {
+    k_shard_kick_fp64(EParams E, const int32_t* F, const int32_t* L, int nf, int ns, int s_lo,
+                      int s_hi) {
     extern __shared__ __align__(16) unsigned char engine_smem[];
     Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
-    for (int ib = ib_lo + (int)blockIdx.x; ib < ib_hi; ib += gridDim.x)
-        kick_unit<HHS_PREC_FP64>(E, F, L, nf, ns, 0.0, ib, 0, 0, nf + ns, sm);
+    const Workers W{(int)blockIdx.x, (int)gridDim.x, kModeGrid};
+    kick_fp64_units(E, F, L, nf, ns, 0.0, nullptr, s_lo, s_hi, nullptr, W, sm);
 }
 
 // v += a*dt for sinks [s_lo, s_hi) from the per-chunk partials (the kick-reduce phase's
@@ -4067,12 +4124,12 @@ hhs_status engine_shard_kick(hhs_ctx* c, const SoA& P, const int32_t* F, const i
     const int blk = engine_shard_kick_block(prec);
     const int nch = pi == 1 ? chunks_host(ntot, eh->grid[1], eh->units_per_cta, kKB) : 1;
     const int C = (ntot + nch - 1) / nch;
+    const int s_lo = b_lo * blk, s_hi = b_hi * blk < ntot ? b_hi * blk : ntot;
     if (pi == 1)
         k_shard_kick_mixed<<<grid, kEB, kEngineSmem, s>>>(E, F, nf, ns, level, nch, C, b_lo, b_hi);
     else
-        k_shard_kick_fp64<<<grid, kEB, kEngineSmem, s>>>(E, F, L, nf, ns, b_lo, b_hi);
+        k_shard_kick_fp64<<<grid, kEB, kEngineSmem, s>>>(E, F, L, nf, ns, s_lo, s_hi);
     HHS_LAUNCH_CHECK();
-    const int s_lo = b_lo * blk, s_hi = b_hi * blk < ntot ? b_hi * blk : ntot;
     const int g2 = (s_hi - s_lo + kEB - 1) / kEB;
     if (pi == 1)
         k_shard_kick_reduce<HHS_PREC_MIXED><<<g2, kEB, 0, s>>>(E, F, L, nf, ns, dt, nch, C, s_lo,

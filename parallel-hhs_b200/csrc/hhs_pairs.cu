@@ -7,6 +7,7 @@
 // src/timestep.cuh:70) and every launch sized from device-resident counts.
 #include "hhs_common.cuh"
 #include "hhs_kernels.h"
+#include "hhs_kick64.cuh"
 #include "hhs_pairmath.cuh"
 
 using namespace hhs;
@@ -262,35 +263,33 @@ __global__ void __launch_bounds__(kKickBlock)
 
 // ---------------------------------------------------------------- standalone kicks
 // kick_slow / kick_sf of the reference API: sinks sink[0..n), sources src[0..m).
-__global__ void __launch_bounds__(kKickBlock)
+// sinks in blocks of 8 up to here (2048 blocks), of 32 beyond: 2.84e11 against 2.66e11 pairs/s
+// at 16384 and 16400 sinks, 3.3e11 at 32768
+constexpr int kK64FineSinks = 16384;
+// FP64: a CTA per block of T = kK64Pairs >> cs sinks, terms evaluated by all its threads and
+// added in source order (hhs_kick64.cuh).
+constexpr int kK64Pairs = 2048;
+__global__ void __launch_bounds__(kK64Threads, 2)
     k_kick_pair_fp64(SoA K, double* __restrict__ ax_out, double* __restrict__ ay_out,
-                     double* __restrict__ az_out, SoA S, int n, int m, double dtfac) {
-    __shared__ double sx[kKickBlock], sy[kKickBlock], sz[kKickBlock], sm[kKickBlock];
-    const int i = blockIdx.x * kKickBlock + threadIdx.x;
-    const bool active = i < n;
-    const double xi = active ? K.x[i] : 0.0, yi = active ? K.y[i] : 0.0,
-                 zi = active ? K.z[i] : 0.0;
-    double ax = 0, ay = 0, az = 0;
-    for (int jt = 0; jt < m; jt += kKickBlock) {
-        const int j = jt + threadIdx.x;
-        if (j < m) {
-            sx[threadIdx.x] = S.x[j]; sy[threadIdx.x] = S.y[j]; sz[threadIdx.x] = S.z[j];
-            sm[threadIdx.x] = S.m[j];
-        }
-        __syncthreads();
-        if (active) {
-            const int jn = min(kKickBlock, m - jt);
-            for (int jl = 0; jl < jn; jl++)
-                kick_pair_fp64(f64_sub(sx[jl], xi), f64_sub(sy[jl], yi), f64_sub(sz[jl], zi), sm[jl],
-                               ax, ay, az);
-        }
-        __syncthreads();
+                     double* __restrict__ az_out, SoA S, int n, int m, double dtfac, int cs) {
+    extern __shared__ __align__(16) unsigned char k64_smem[];
+    auto& k = *reinterpret_cast<Kick64Smem<kK64Pairs>*>(k64_smem);
+    const int T = kK64Pairs >> cs, s0 = blockIdx.x * T, nsink = min(T, n - s0);
+    const int tid = threadIdx.x;
+    if (tid < nsink) {
+        k.sx[tid] = K.x[s0 + tid]; k.sy[tid] = K.y[s0 + tid]; k.sz[tid] = K.z[s0 + tid];
     }
-    if (!active) return;
-    if (ax_out) { ax_out[i] = ax; ay_out[i] = ay; az_out[i] = az; }
-    K.vx[i] = f64_add(K.vx[i], f64_mul(ax, dtfac));
-    K.vy[i] = f64_add(K.vy[i], f64_mul(ay, dtfac));
-    K.vz[i] = f64_add(K.vz[i], f64_mul(az, dtfac));
+    __syncthreads();
+    const double a = kick64_sums(k, cs, nsink, m, 0.0, [](int j) { return j; },
+                                 [&](int j, double& x, double& y, double& z, double& mj) {
+                                     x = S.x[j]; y = S.y[j]; z = S.z[j]; mj = S.m[j];
+                                 });
+    const int c = tid / T, i = s0 + (tid & (T - 1));
+    if (c >= 3 || i >= n) return;
+    double* out = c == 0 ? ax_out : (c == 1 ? ay_out : az_out);
+    double* v = c == 0 ? K.vx : (c == 1 ? K.vy : K.vz);
+    if (out) out[i] = a;
+    v[i] = f64_add(v[i], f64_mul(a, dtfac));
 }
 
 __global__ void __launch_bounds__(kKickBlock)
@@ -441,10 +440,14 @@ hhs_status launch_kick_pair(const SoA& sink, double* ax, double* ay, double* az,
                             const SoA& src, int n_sink, int n_src, double dtfac,
                             hhs_precision prec, cudaStream_t stream) {
     if (n_sink <= 0) return HHS_OK;
-    if (prec == HHS_PREC_FP64)
-        k_kick_pair_fp64<<<grid_for(n_sink, kKickBlock), kKickBlock, 0, stream>>>(
-            sink, ax, ay, az, src, n_sink, n_src, dtfac);
-    else
+    if (prec == HHS_PREC_FP64) {
+        const int cs = n_sink <= kK64FineSinks ? 8 : 6;
+        constexpr int bytes = (int)sizeof(Kick64Smem<kK64Pairs>);
+        HHS_CUDA_TRY(cudaFuncSetAttribute(k_kick_pair_fp64,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        k_kick_pair_fp64<<<grid_for(n_sink, kK64Pairs >> cs), kK64Threads, bytes, stream>>>(
+            sink, ax, ay, az, src, n_sink, n_src, dtfac, cs);
+    } else
         k_kick_pair_mixed<<<grid_for(n_sink, kKickBlock), kKickBlock, 0, stream>>>(
             sink, ax, ay, az, src, n_sink, n_src, dtfac);
     HHS_LAUNCH_CHECK();
