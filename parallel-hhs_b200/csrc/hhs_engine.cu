@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include <algorithm>
+#include <array>
 #include <cstddef>
 #include <cstdint>
 #include <new>
@@ -51,6 +52,7 @@ constexpr int kKB = 2 * kEB;      // sinks per block of the mixed grid kick (two
 constexpr int kTS = 1024;         // source records per shared-memory tile of that kick
 constexpr int kTX = 256;          // slow records per tile of the symmetric grid kick
 constexpr int kTW = 256;          // widest column tile of the packed grid timestep
+constexpr int kTfCap = 2048;      // pairs that a filtered timestep lists at a time
 constexpr int kMaxFsb = 64;       // fast super-blocks of that kick (column-partial slots)
 constexpr int kMaxChunks = 32;    // source chunks per node (partial-sum slots)
 constexpr int kK64Pairs = 2048;   // pair terms per stage of the FP64 kick
@@ -63,7 +65,7 @@ enum ProfKind {
 
 struct EngineState {
     unsigned bar_count;   // grid-barrier arrivals of this launch (cleared before each launch)
-    unsigned bar_gen;
+    unsigned m_max;       // largest |mass| of the launch's system (FP32 bits, cleared likewise)
     unsigned pad[2];
     unsigned kick_ctr[2][kMaxLevels];  // dynamic work counters of each level's kick units
     unsigned long long prof_ns[8];
@@ -107,6 +109,11 @@ struct EParams {
     // of entry p: (x hi, y hi), (z hi, mass), (x lo, y lo), (z lo, vx), (vy, vz)
     float4* tq;
     long long tq_stride;
+    // the same members for the filtered timestep: entry p holds members 2p and 2p + 1 as five
+    // float4 (x, y), (z, vx), (vy, vz), (|x|^2 - a, |v|^2), (-kappa, -b), see tf_put
+    float4* tf;
+    unsigned long long* tau_key;  // [n_max] FP64: complement of the least pair timescale's bits
+    int filter;      // grid nodes below the top one filter their pairs (tf_row)
     int prec_mixed;  // this launch runs the mixed-precision kernels
     int overlap;     // slow-only kick units beside a subtree's first pass (tuning)
     int4* trace;                        // node record {level, n, n_fast, calc} in call order
@@ -172,6 +179,9 @@ struct __align__(16) Smem {
     int bcast;
     unsigned bar_k;               // grid barriers passed by this CTA in this launch
     unsigned epoch;               // look-back epoch of the current split
+    unsigned tf_cnt;              // filtered timestep: passing pairs, of which
+    int tf_n;                     // tf_n are listed, and the first unit that overflowed the
+    long long tf_ov;              // list (-1: none)
     unsigned kphase;              // parity of the next phase of kbar
     unsigned tphase;              // parities of the next phases of tbar[0], tbar[1]
     __align__(8) uint64_t kbar;   // completion barrier of the kick's source-tile copies
@@ -192,6 +202,10 @@ struct __align__(16) Smem {
             float4 Q[2][5][kTW / 2];                              // column pairs
             float colred[2][kEB / 32][kTW];
         } ts2;
+        struct {                                                  // filtered timestep
+            float4 T[2][kTW / 2][5];                              // column pairs
+            int2 hit[kTfCap];                                     // passing pairs
+        } tf;
         struct { float4 P0[kEB], P1[kEB], P2[kEB]; float2 M[kEB]; } kx;  // packed kick tiles
         Kick64Smem<kK64Pairs> k64;                              // FP64 kick terms
         struct {                                                  // tiny-subtree state
@@ -204,6 +218,11 @@ struct __align__(16) Smem {
         } tiny;
     } u;
 };
+
+// The CTA's Smem, for functions that are not inlined into their kernel: a reference passed to
+// them would be a generic pointer, and every shared-memory read a generic load.
+extern __shared__ __align__(16) unsigned char dyn_smem[];
+__device__ __forceinline__ Smem& cta_smem() { return *reinterpret_cast<Smem*>(dyn_smem); }
 
 // dynamic shared memory of the persistent kernel: Smem with its last member grown to
 // hold a MidState
@@ -654,15 +673,6 @@ __device__ __forceinline__ TsSink2 tq_sink(const EParams& E, int i) {
                    f2dup(-q[4 * a]), f2dup(-q[4 * a + 2]), f2dup(q[a + 2])};
 }
 
-// The node's members (list S, n of them) into the packed timestep arrays.
-__device__ void pack_ts(const EParams& E, const int32_t* S, int n, const Workers& W) {
-    const SoA& P = E.P;
-    for (int i = W.id * kEB + (int)threadIdx.x; i < n; i += W.count * kEB) {
-        const int g = list_at(S, i);
-        tq_put(E, i, P.x[g], P.y[g], P.z[g], P.m[g], P.vx[g], P.vy[g], P.vz[g]);
-    }
-}
-
 // unit u of the triangle -> (row block, column block)
 __device__ __forceinline__ void ts_tile_of(long long u, int nrb, int ncb, int step, int& rb,
                                            int& cb) {
@@ -685,8 +695,8 @@ __device__ __forceinline__ void ts_tile_stage(const EParams& E, int buf, int c0,
                   &sm.tbar[buf]);
 }
 
-__device__ void ts_sym_tiles(const EParams& E, int n, int cw, long long u0, long long u1,
-                             Smem& sm) {
+__device__ void ts_sym_tiles(const EParams& E, int n, int cw, long long u0, long long u1) {
+    Smem& sm = cta_smem();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int step = kEB / cw;
     const int nrb = (n + kEB - 1) / kEB, ncb = (n + cw - 1) / cw;
@@ -786,6 +796,363 @@ __device__ void ts_sym_tiles(const EParams& E, int n, int cw, long long u0, long
     __syncthreads();  // colred and the buffers are free; every wait of this range is done
     if (threadIdx.x == 0) sm.tphase = phase;
     __syncthreads();
+}
+
+// ---------------------------------------------------------------- filtered grid timestep
+// A particle's timestep is the least of its pair timescales (src/timestep.cuh:27-57), its rate
+// R = 1 / timestep the greatest of its pair rates, and only one pair in thousands comes near
+// it. So a node below the top one does not evaluate its pairs: it guesses a lower bound T of
+// each rate from the timestep that the particle has (computed earlier in this launch, at most
+// a few per cent off, since a particle moves for at most its timestep in between), passes over
+// all pairs with a test that no pair above T fails, and evaluates the few that pass exactly as
+// the full evaluation does. The split then checks that a rate of at least T was found; where
+// it was not (the guess was too high), it scans that row whole. So the result is the maximum
+// over all pairs bit for bit, whatever the guesses.
+//
+// The test. With r, w the distance and the speed over the distance, M the mass sum and
+// rate_ff, rate_fb the free-fall and fly-by rates as ts_pair_rate_mixed has them,
+//     rate_ff <= sqrt(2 M / r^3) / eta + 3/4 w,
+//     rate_fb <= (1 / eta + 1/2) w + M / (2 |dv| r^2).
+// Let e = 1 / eta + 1/2, A = r^2, B = |dv|^2. If A >= kappa B + a and B >= b with
+//     kappa = (e / (alpha T))^2, a = (2 M / (eta beta T)^2)^(2/3), beta = 1 - 3/4 alpha / e,
+//     b = (M / (2 (1 - alpha) T a))^2,
+// then w <= alpha T / e, so rate_ff <= beta T + 3/4 alpha T / e = T and rate_fb <= alpha T +
+// (1 - alpha) T = T. (eta <= 1 keeps beta above 1/2.) M is bounded by m_i + m_max. T is taken 1%
+// lower than guessed, which covers the rounding of the pair rates themselves. An unordered
+// pair is tested once for both its particles, with max(kappa_i, kappa_j), a_i + a_j and
+// b_i + b_j.
+//
+// Both squares come from dot products, A = |x_i|^2 + |x_j|^2 - 2 x_i x_j: 9 packed operations
+// for two pairs, where their rates take about a hundred instructions. Rounding (below 1.5e-6 of
+// |x_i|^2 + |x_j|^2) is covered by shrinking the |x|^2 and growing the |v|^2 by 4e-6, which
+// keeps the computed A below and B above the true ones, and by a margin in b.
+// Measured: the timestep phases of an N=65536 step (Salpeter masses) 123.0 -> 41 ms, 16384 4.10 ->
+// 2.24 (FP64: 40.7 -> 2.6); a calc of 64678 members 1.21 ms, 1.7e12 unordered pairs/s. What
+// bounds it: the FMA pipe (half busy) and, below about 6000 members, the latency of the tiles.
+constexpr float kTfAlpha = 0.8f;
+// T over the old rate: at 0.7 the larger kappa costs 7% of the calcs at N=16384, at 0.85 a few
+// rows a step are scanned whole (150 us a step)
+constexpr double kTfGuess = 0.8;
+constexpr float kTfAll = 1.0e38f;   // a particle whose pairs all pass
+
+// The lower bound of member i's rate that the filter uses (0: none, every pair passes): from
+// the full FP32 evaluation (FP64, top node) or from its old timestep.
+template <int PREC>
+__device__ __forceinline__ double tf_bound(const EParams& E, int i, int g, bool top) {
+    const double t = PREC == HHS_PREC_FP64 && top
+                         ? 0.999 * (double)__uint_as_float(__ldcg(&E.rate_acc[i]))
+                         : kTfGuess / E.P.ts[g];
+    return t > 1e-12 && t < 1e12 ? t : 0.0;
+}
+
+// Member i for the filter, bound as tf_bound gives it: component i & 1 of its entry.
+__device__ __forceinline__ void tf_put(const EParams& E, int i, double x, double y, double z,
+                                       double vx, double vy, double vz, double mass,
+                                       double bound) {
+    const double r2 = x * x + y * y + z * z, v2 = vx * vx + vy * vy + vz * vz;
+    const float T = 0.99f * (float)bound, eta = (float)E.eta;
+    const float M = (float)fabs(mass) + __uint_as_float(__ldcg(&E.st->m_max));
+    const float e = 1.0f / eta + 0.5f, beta = 1.0f - 0.75f * kTfAlpha / e;
+    const float k = e / (kTfAlpha * T), kappa = 1.01f * k * k;
+    const float f = eta * beta * T, c = cbrtf(2.01f * M / (f * f)), a = 1.02f * c * c + 1e-30f;
+    const float h = 0.5f * M / ((1.0f - kTfAlpha) * T * a);
+    // false for NaN; without it every pair of the member passes
+    const bool ok = r2 < 1e24 && v2 < 1e24 && bound > 0.0 && kappa < 1e24f && a < 1e24f && h < 1e12f;
+    float* q = reinterpret_cast<float*>(E.tf) + 20 * (size_t)(i >> 1) + (i & 1);
+    q[0] = ok ? (float)x : 0.0f;
+    q[2] = ok ? (float)y : 0.0f;
+    q[4] = ok ? (float)z : 0.0f;
+    q[6] = ok ? (float)vx : 0.0f;
+    q[8] = ok ? (float)vy : 0.0f;
+    q[10] = ok ? (float)vz : 0.0f;
+    q[12] = ok ? (float)(r2 * (1.0 - 4e-6) - 1.001 * (double)a) : -kTfAll;
+    q[14] = ok ? (float)(v2 * (1.0 + 4e-6)) : 0.0f;
+    q[16] = ok ? -kappa : 0.0f;
+    q[18] = ok ? -(1.02f * h * h + 4e-5f * (float)v2 + 1e-30f) : 0.0f;
+}
+
+struct TfRow {
+    float2 x, y, z, vx, vy, vz, U;  // -2 x, -2 v, |v|^2, each in both lanes
+    float nk, c1, c2;               // -kappa; pass: v <= c1 or B - b_j < c2
+};
+
+__device__ __forceinline__ TfRow tf_row(const float4* tf, int i) {
+    const float* q = reinterpret_cast<const float*>(tf) + 20 * (size_t)(i >> 1) + (i & 1);
+    TfRow r;
+    r.x = f2dup(-2.0f * q[0]);
+    r.y = f2dup(-2.0f * q[2]);
+    r.z = f2dup(-2.0f * q[4]);
+    r.vx = f2dup(-2.0f * q[6]);
+    r.vy = f2dup(-2.0f * q[8]);
+    r.vz = f2dup(-2.0f * q[10]);
+    r.U = f2dup(q[14]);
+    r.nk = q[16];
+    r.c1 = -q[12];
+    r.c2 = -q[18];
+    return r;
+}
+
+// Tests of two columns (one packed entry) for a row: v = A - max(kappa) B - a_i - a_j less the
+// row's own |x|^2 - a, and B - b_j.
+__device__ __forceinline__ void tf_test(const float4 (&Q)[5], const TfRow& r, float2& v,
+                                        float2& B) {
+    B = __ffma2_rn(r.vx, make_float2(Q[1].z, Q[1].w), make_float2(Q[3].z, Q[3].w));
+    B = __ffma2_rn(r.vy, make_float2(Q[2].x, Q[2].y), B);
+    B = __ffma2_rn(r.vz, make_float2(Q[2].z, Q[2].w), B);
+    B = __fadd2_rn(B, r.U);
+    v = __ffma2_rn(r.x, make_float2(Q[0].x, Q[0].y), make_float2(Q[3].x, Q[3].y));
+    v = __ffma2_rn(r.y, make_float2(Q[0].z, Q[0].w), v);
+    v = __ffma2_rn(r.z, make_float2(Q[1].x, Q[1].y), v);
+    v = __ffma2_rn(make_float2(fminf(r.nk, Q[4].x), fminf(r.nk, Q[4].y)), B, v);
+    B = __fadd2_rn(B, make_float2(Q[4].z, Q[4].w));
+}
+
+// The exact pair rate (mixed) or timescale (FP64) of particles gi, gj, merged into *best.
+__device__ __forceinline__ float tf_rate(const EParams& E, int gi, int gj) {
+    const SoA& P = E.P;
+    const DS xi = ds_split(P.x[gi]), yi = ds_split(P.y[gi]), zi = ds_split(P.z[gi]);
+    const DS xj = ds_split(P.x[gj]), yj = ds_split(P.y[gj]), zj = ds_split(P.z[gj]);
+    return ts_pair_rate_mixed(ds_diff(xi.hi, xi.lo, xj.hi, xj.lo),
+                              ds_diff(yi.hi, yi.lo, yj.hi, yj.lo),
+                              ds_diff(zi.hi, zi.lo, zj.hi, zj.lo),
+                              (float)P.vx[gi] - (float)P.vx[gj], (float)P.vy[gi] - (float)P.vy[gj],
+                              (float)P.vz[gi] - (float)P.vz[gj], (float)P.m[gi] + (float)P.m[gj],
+                              E.inv_eta_s2, E.inv_eta);
+}
+__device__ __forceinline__ double tf_tau(const EParams& E, int gi, int gj) {
+    const SoA& P = E.P;
+    double t = 1.e30;
+    ts_pair_fp64(f64_sub(P.x[gi], P.x[gj]), f64_sub(P.y[gi], P.y[gj]), f64_sub(P.z[gi], P.z[gj]),
+                 f64_sub(P.vx[gi], P.vx[gj]), f64_sub(P.vy[gi], P.vy[gj]),
+                 f64_sub(P.vz[gi], P.vz[gj]), P.m[gi], P.m[gj], E.eta, E.eta_s2, t);
+    return t;
+}
+template <int PREC>
+__device__ __forceinline__ void tf_merge(const EParams& E, const int32_t* S, int i, int j) {
+    const int gi = list_at(S, i), gj = list_at(S, j);
+    if constexpr (PREC == HHS_PREC_FP64) {
+        const double t = tf_tau(E, gi, gj);
+        if (t < 1.e30) {
+            const unsigned long long key = ~(unsigned long long)__double_as_longlong(t);
+            atomicMax(&E.tau_key[i], key);
+            atomicMax(&E.tau_key[j], key);
+        }
+    } else {
+        const float r = tf_rate(E, gi, gj);
+        if (r > 0.0f) {
+            atomicMax(&E.rate_acc[i], __float_as_uint(r));
+            atomicMax(&E.rate_acc[j], __float_as_uint(r));
+        }
+    }
+}
+
+// Tiles of a node: the upper triangle of (rbn-row, cw-column) blocks, row-major. Rows: 512 in
+// large nodes; smaller blocks divide better over the workers (with 512 rows from 8192 members
+// on, 256 from 4096, a calc of 14811 or 13271 members takes 10% more; with 512 rows throughout,
+// one of 1622 takes 12.5 us instead of 10.7). Columns as wide as still gives every worker two
+// units.
+constexpr int kTfRows512 = 16384, kTfRows256 = 2048;
+__device__ __forceinline__ long long tf_units(int n, int rbn, int cw) {
+    const long long nrb = (n + rbn - 1) / rbn, ncb = (n + cw - 1) / cw;
+    return nrb * ncb - rbn / cw * (nrb * (nrb - 1) / 2);
+}
+__device__ __forceinline__ int tf_rows(int n) { return n >= kTfRows512 ? 512 : (n >= kTfRows256 ? 256 : 128); }
+__device__ __forceinline__ int tf_tile_width(int n, int rbn, int workers) {
+    int cw = min(kTW, rbn);
+    while (cw > 32 && tf_units(n, rbn, cw) < 2LL * workers) cw >>= 1;
+    return cw;
+}
+
+// Units [u0, u1) of the node's (rbn-row, cw-column) tiles until the list of passing pairs
+// (shared memory) is half full; returns the next unit. A thread tests two rows of the row block
+// (each shared-memory read serves both) against the columns of its group: 512 rows and one
+// group, or fewer rows and their columns divided over 2 or 4 groups. Each unit's columns arrive
+// by bulk copy while the previous unit computes. sm.tf_n pairs are listed; if the list
+// overflowed, it holds those of the units before sm.tf_ov, and every pair of the units from
+// there on is taken to pass.
+__device__ __forceinline__ long long ts_filter_tiles(const EParams& E, int n, int rbn, int cw,
+                                                     long long u0, long long u1, Smem& sm) {
+    auto& F = sm.u.tf;
+    const int tid = threadIdx.x, ncb = (n + cw - 1) / cw, step = rbn / cw;
+    const int half = rbn >> 1, r0 = tid & (half - 1), grp = tid / half, ngrp = kEB / half;
+    int rb = 0, cb = 0;
+    ts_tile_of(u0, (n + rbn - 1) / rbn, ncb, step, rb, cb);
+    int rb2 = rb, cb2 = cb;  // the next unit to copy
+    long long staged = u0;
+    auto stage = [&]() {
+        const int buf = (int)(staged - u0) & 1;
+        const int c0 = cb2 * cw, np = (min(cw, n - c0) + 1) >> 1;
+        if (tid == 0) {
+            mbar_arrive_expect_tx(&sm.tbar[buf], (unsigned)np * 80u);
+            bulk_load(F.T[buf], E.tf + 5 * (size_t)(c0 >> 1), (unsigned)np * 80u, &sm.tbar[buf]);
+        }
+        if (++cb2 >= ncb) { rb2++; cb2 = rb2 * step; }
+        staged++;
+    };
+    if (tid == 0) {
+        sm.tf_cnt = 0u;
+        sm.tf_ov = -1;
+    }
+    stage();
+    if (staged < u1) stage();
+    unsigned phase = sm.tphase, held = 0u;
+    int cur = -1;
+    TfRow row[2];
+    __syncthreads();
+    long long u = u0;
+    for (; u < staged; u++) {
+        const int buf = (int)(u - u0) & 1;
+        const int c0 = cb * cw, np = (min(cw, n - c0) + 1) >> 1;
+        if (rb != cur) {
+            cur = rb;
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int i = rb * rbn + r * half + r0;
+                row[r] = tf_row(E.tf, min(i, n - 1));
+                if (i >= n) row[r].c1 = row[r].c2 = -3e38f;  // no pair passes
+            }
+        }
+        if (!mbar_wait(&sm.tbar[buf], (phase >> buf) & 1u, E.err))
+            (void)mbar_wait(&sm.tbar[buf], (phase >> buf) & 1u, nullptr);
+        phase ^= 1u << buf;
+        const float4(*T)[5] = F.T[buf];
+        const int pe = (np * (grp + 1)) / ngrp;
+        for (int p0 = (np * grp) / ngrp; p0 < pe; p0 += 2) {
+            __syncwarp();  // lanes that listed pairs rejoin the others here, not later
+            const int p1 = min(p0 + 1, pe - 1);
+            bool any = false;
+            float2 va[2], Ba[2], vb[2], Bb[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++) tf_test(T[p0], row[r], va[r], Ba[r]);
+#pragma unroll
+            for (int r = 0; r < 2; r++) tf_test(T[p1], row[r], vb[r], Bb[r]);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const float mv = fminf(fminf(va[r].x, va[r].y), fminf(vb[r].x, vb[r].y));
+                const float mB = fminf(fminf(Ba[r].x, Ba[r].y), fminf(Bb[r].x, Bb[r].y));
+                any = any || mv <= row[r].c1 || mB < row[r].c2;
+            }
+            if (any) {
+#pragma unroll 1
+                for (int p = p0; p <= p1; p++) {
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        float2 v, B;
+                        tf_test(T[p], row[r], v, B);
+                        const int i = rb * rbn + r * half + r0, j = c0 + 2 * p;
+                        const bool h0 = (v.x <= row[r].c1 || B.x < row[r].c2) && j > i;
+                        const bool h1 = (v.y <= row[r].c1 || B.y < row[r].c2) && j + 1 > i &&
+                                        j + 1 < n;
+                        const unsigned cnt = (h0 ? 1u : 0u) + (h1 ? 1u : 0u);
+                        if (cnt) {
+                            const unsigned k = atomicAdd(&sm.tf_cnt, cnt);
+                            if (h0 && k < kTfCap) F.hit[k] = make_int2(i, j);
+                            if (h1 && k + cnt - 1 < kTfCap) F.hit[k + cnt - 1] = make_int2(i, j + 1);
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();  // this buffer's columns are read, the list is complete
+        const unsigned cnt = sm.tf_cnt;
+        if (cnt > kTfCap && held <= kTfCap) {  // the first unit of an overflow
+            if (tid == 0) {
+                sm.tf_ov = u;
+                sm.tf_n = (int)held;
+            }
+            held = kTfCap + 1;
+        } else if (held <= kTfCap) {
+            held = cnt;
+        }
+        if (cnt <= kTfCap / 2 && staged < u1) stage();
+        __syncthreads();  // every thread has the count: the next unit may add to it
+        if (++cb >= ncb) { rb++; cb = rb * step; }
+    }
+    if (tid == 0) {
+        sm.tphase = phase;
+        if (held <= kTfCap) sm.tf_n = (int)held;
+    }
+    __syncthreads();
+    return u;
+}
+
+// Evaluates what ts_filter_tiles listed, up to its unit u1.
+template <int PREC>
+__device__ __forceinline__ void ts_filter_merge(const EParams& E, const int32_t* S, int n, int rbn,
+                                                int cw, long long u1, Smem& sm) {
+    const int ncb = (n + cw - 1) / cw;
+    const int listed = sm.tf_n;
+    const long long per = (long long)rbn * cw, all = sm.tf_ov >= 0 ? (u1 - sm.tf_ov) * per : 0;
+    for (long long k = threadIdx.x; k < listed + all; k += kEB) {
+        int2 h;
+        if (k < listed) {
+            h = sm.u.tf.hit[k];
+        } else {
+            const long long q = (k - listed) / per;
+            const int w = (int)((k - listed) - q * per);
+            int rb, cb;
+            ts_tile_of(sm.tf_ov + q, (n + rbn - 1) / rbn, ncb, rbn / cw, rb, cb);
+            h = make_int2(rb * rbn + w / cw, cb * cw + w % cw);
+            if (h.x >= n || h.y >= n || h.y <= h.x) continue;
+        }
+        tf_merge<PREC>(E, S, h.x, h.y);
+    }
+    __syncthreads();  // the list is read
+}
+
+// The node's members (list S, n of them) into the packed arrays of the full evaluation, and
+// their largest |mass| into m_max.
+__device__ void pack_ts(const EParams& E, const int32_t* S, int n, const Workers& W) {
+    const SoA& P = E.P;
+    float mm = 0.0f;
+    for (int i = W.id * kEB + (int)threadIdx.x; i < n; i += W.count * kEB) {
+        const int g = list_at(S, i);
+        tq_put(E, i, P.x[g], P.y[g], P.z[g], P.m[g], P.vx[g], P.vy[g], P.vz[g]);
+        mm = fmaxf(mm, __double2float_ru(fabs(P.m[g])));
+    }
+    const unsigned b = __reduce_max_sync(HHS_FULL_MASK, __float_as_uint(mm));
+    if ((threadIdx.x & 31) == 0 && b) atomicMax(&E.st->m_max, b);
+}
+
+// The same for the filter.
+template <int PREC>
+__device__ void pack_tf(const EParams& E, const int32_t* S, int n, bool top, const Workers& W) {
+    const SoA& P = E.P;
+    for (int i = W.id * kEB + (int)threadIdx.x; i < n; i += W.count * kEB) {
+        const int g = list_at(S, i);
+        tf_put(E, i, P.x[g], P.y[g], P.z[g], P.vx[g], P.vy[g], P.vz[g], P.m[g],
+               tf_bound<PREC>(E, i, g, top));
+    }
+}
+
+// The whole pair row of member `i` by the calling warp: its greatest rate (mixed) or least
+// timescale (FP64), for a row whose bound was too high.
+template <int PREC>
+__device__ double tf_scan_row(const EParams& E, const int32_t* S, int n, int i) {
+    const int lane = threadIdx.x & 31, gi = list_at(S, i);
+    double best = PREC == HHS_PREC_FP64 ? 1.e30 : 0.0;
+    int g[4];
+    for (int j0 = lane; j0 < n; j0 += 128) {  // four pairs in flight
+#pragma unroll
+        for (int k = 0; k < 4; k++) g[k] = j0 + 32 * k < n ? list_at(S, j0 + 32 * k) : gi;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (g[k] == gi) continue;
+            if (PREC == HHS_PREC_FP64) {
+                const double t = tf_tau(E, gi, g[k]);
+                best = t < best ? t : best;
+            } else {
+                const float r = tf_rate(E, gi, g[k]);
+                best = (double)r > best ? (double)r : best;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double b = __shfl_xor_sync(HHS_FULL_MASK, best, o);
+        best = PREC == HHS_PREC_FP64 ? (b < best ? b : best) : (b > best ? b : best);
+    }
+    return best;
 }
 
 // ---------------------------------------------------------------- FP64 kick units
@@ -1868,9 +2235,10 @@ __device__ void scatter_phase(const EParams& E, const int32_t* S, int n, double 
 // which is the lone particle's place after the fold and an unused slot otherwise (every
 // slow particle lands below n-1 once one fast particle exists). The tile that ends the
 // list writes the counts and the work counters.
-template <int PREC>
+template <int PREC, bool FILTER>
 __device__ void split_phase(const EParams& E, const int32_t* S, int n, double dt, int level,
-                            bool calc, int nch, const Workers& W, Smem& sm) {
+                            bool calc, int nch, bool filtered, bool top, const Workers& W,
+                            Smem& sm) {
     const int ntiles = (n + kEB - 1) / kEB;
     int32_t* F = E.fast_lists + (size_t)level * E.n_max;
     int32_t* L = E.slow_lists + (size_t)level * E.n_max;
@@ -1880,10 +2248,26 @@ __device__ void split_phase(const EParams& E, const int32_t* S, int n, double dt
     for (int t = W.id; t < ntiles; t += W.count) {
         const int i = t * kEB + threadIdx.x;
         int flag = 0, gi = 0;
+        double ts = 0.0;
         if (i < n) {
             gi = list_at(S, i);
-            double ts;
-            if (calc) {
+            if (FILTER && calc && filtered) {
+                // a rate of at least the bound that the filter used was found, or the row is
+                // scanned below
+                const double bound = tf_bound<PREC>(E, i, gi, top);
+                if (PREC == HHS_PREC_FP64) {
+                    ts = __longlong_as_double((long long)~E.tau_key[i]);
+                    if (!(ts < 1.e30)) ts = 1.e30;  // no pair (the key's complement is a NaN)
+                    E.tau_key[i] = 0ull;
+                    flag = ts * bound > 1.0;
+                } else {
+                    const float mr = __uint_as_float(E.rate_acc[i]);
+                    const double tv = 1.0 / (double)mr;
+                    ts = tv < 1.e30 ? tv : 1.e30;
+                    flag = (double)mr < bound;
+                }
+                E.rate_acc[i] = 0u;
+            } else if (calc) {
                 if (PREC == HHS_PREC_FP64) {
                     double mv = 1.e30;
                     for (int c = 0; c < nch; c++) {
@@ -1897,12 +2281,22 @@ __device__ void split_phase(const EParams& E, const int32_t* S, int n, double dt
                     const double tv = 1.0 / (double)mr;
                     ts = tv < 1.e30 ? tv : 1.e30;
                 }
-                E.P.ts[gi] = ts;
             } else {
                 ts = E.P.ts[gi];
             }
-            flag = ts <= dt;
         }
+        if (FILTER && calc && filtered) {
+            for (unsigned bad = __ballot_sync(HHS_FULL_MASK, flag); bad; bad &= bad - 1u) {
+                const int l = __ffs(bad) - 1;
+                const double best = tf_scan_row<PREC>(E, S, n, (i & ~31) + l);
+                if ((i & 31) == l) {
+                    const double tv = PREC == HHS_PREC_FP64 ? best : 1.0 / best;
+                    ts = tv < 1.e30 ? tv : 1.e30;
+                }
+            }
+        }
+        if (i < n && calc) E.P.ts[gi] = ts;
+        flag = i < n && ts <= dt;
         int tot;
         const int ex = block_excl_flag(flag, sm, tot);
         if (threadIdx.x < 32) {
@@ -1968,7 +2362,7 @@ __device__ void split_phase(const EParams& E, const int32_t* S, int n, double dt
 // thread per sink (slow then fast sources, the reference's order).
 // nfsb >= 0: the symmetric kick's partials (nch = its chunk count: fast sinks add their
 // nch chunk partials, slow sinks those and then their nfsb super-block partials).
-template <int PREC>
+template <int PREC, bool FILTER>
 __device__ void kick_reduce_phase(const EParams& E, const int32_t* F, const int32_t* L, int nf,
                                   int ns, double dt, int nch, int C, const Workers& W,
                                   Smem& sm, int nfsb = -1) {
@@ -1992,6 +2386,9 @@ __device__ void kick_reduce_phase(const EParams& E, const int32_t* F, const int3
                 v1[k] = v;
             }
             P.vx[g] = v1[0]; P.vy[g] = v1[1]; P.vz[g] = v1[2];
+            if (FILTER && !slow && E.filter && W.mode == kModeGrid)
+                tf_put(E, s, P.x[g], P.y[g], P.z[g], v1[0], v1[1], v1[2], P.m[g],
+                       tf_bound<PREC>(E, s, g, false));
             if (slow) {
                 P.x[g] = f64_add(f64_add(P.x[g], f64_mul(v0[0], h)), f64_mul(v1[0], h));
                 P.y[g] = f64_add(f64_add(P.y[g], f64_mul(v0[1], h)), f64_mul(v1[1], h));
@@ -2041,7 +2438,11 @@ __device__ void kick_reduce_phase(const EParams& E, const int32_t* F, const int3
                 P.vx[g] = v1[0]; P.vy[g] = v1[1]; P.vz[g] = v1[2];
                 if (!slow && E.tq && W.mode == kModeGrid) {
                     // the fast set's next pass recomputes its timesteps from these records
-                    tq_put(E, s2, P.x[g], P.y[g], P.z[g], P.m[g], v1[0], v1[1], v1[2]);
+                    if (FILTER && E.filter)
+                        tf_put(E, s2, P.x[g], P.y[g], P.z[g], v1[0], v1[1], v1[2], P.m[g],
+                               tf_bound<PREC>(E, s2, g, false));
+                    else
+                        tq_put(E, s2, P.x[g], P.y[g], P.z[g], P.m[g], v1[0], v1[1], v1[2]);
                 }
                 if (slow) {
                     P.x[g] = fma(v1[0], h, fma(v0[0], h, P.x[g]));
@@ -2817,8 +3218,9 @@ __device__ void warp_subtree(const EParams& E, MidState& M, const unsigned* memw
 // cs, rank: the hardware cluster that runs the subtree (every CTA of it calls mid_hold),
 // or cs = 1 for one CTA alone whatever cluster it belongs to.
 template <int PREC>
-__device__ void mid_hold(const EParams& E, const int32_t* S, int n, int level0, bool calc0,
-                         int dist_n, int cs, int rank, Smem& sm) {
+__device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int n, int level0, bool calc0,
+                         int dist_n, int cs, int rank) {
+    Smem& sm = cta_smem();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     MidState& M = *reinterpret_cast<MidState*>(&sm.u);
@@ -3155,7 +3557,7 @@ __device__ __forceinline__ bool kick_overlaps(const EParams& E, int lvl, const W
 // Walks the HOLD recursion from `top` (whose subsystem is already defined by the
 // counts/lists above it). Grid and cluster modes delegate nodes with n <= small_n,
 // with their whole subtree, to worker 0 alone.
-template <int PREC, int MODE>
+template <int PREC, int MODE, bool FILTER>
 __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers& W, Smem& sm,
                          unsigned long long& t_last) {
     unsigned long long after1 = 0, after2 = 0, calcm = 0;  // per-level state bits
@@ -3182,7 +3584,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     const int cs = (int)cg::this_cluster().num_blocks();
                     if ((int)blockIdx.x < cs) {
                         mid_hold<PREC>(E, S, n, lvl, calc, E.mid_dist_n, cs,
-                                       (int)cg::this_cluster().block_rank(), sm);
+                                       (int)cg::this_cluster().block_rank());
                     } else if (!calc && lvl > top && kick_overlaps(E, lvl - 1, W)) {
                         // meanwhile the other CTAs run the parent's kick units that do not
                         // involve the fast set (this node), which mid_hold is advancing
@@ -3193,7 +3595,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                                        1, sm);
                     }
                 } else {
-                    mid_hold<PREC>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id, sm);
+                    mid_hold<PREC>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfCluster, 0.0, sm, lvl);
@@ -3213,7 +3615,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 if (W.id == 0) {
                     const Workers one{0, 1, kModeBlock};
                     unsigned long long t_sub = 0;
-                    run_hold<PREC, kModeBlock>(E, lvl, calc, one, sm, t_sub);
+                    run_hold<PREC, kModeBlock, false>(E, lvl, calc, one, sm, t_sub);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfSubtree, 0.0, sm, lvl);
@@ -3222,8 +3624,41 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 continue;
             }
             int nch = 1;
+            bool filtered = false;
             if (calc) {
-                if (PREC == HHS_PREC_FP64) {
+                const bool filter = FILTER && E.filter;
+                if (MODE == kModeGrid && (filter || (PREC != HHS_PREC_FP64 && E.tq))) {
+                    // Members are packed by the parent's kick-reduce phase, or here when it had
+                    // no kick and in the top node. The top node has no timesteps to guess from:
+                    // it evaluates every pair's FP32 rate, and filters only to get FP64.
+                    const bool top_node = lvl == top;
+                    const bool pack = top_node || ld_volatile_i32(&E.counts[lvl - 1].n_slow) == 0;
+                    filtered = filter && (!top_node || PREC == HHS_PREC_FP64);
+                    if (!filter || top_node) {
+                        if (pack) {
+                            pack_ts(E, S, n, W);
+                            if (!phase_barrier(E, sm, W)) return false;
+                        }
+                        const int cw = ts_tile_width(n, W.count);
+                        const long long units = ts_tile_units(n, cw);
+                        ts_sym_tiles(E, n, cw, units * W.id / W.count,
+                                     units * (W.id + 1) / W.count);
+                        if (filtered && !phase_barrier(E, sm, W)) return false;
+                    }
+                    if (FILTER && filtered) {
+                        if (pack) {
+                            pack_tf<PREC>(E, S, n, top_node, W);
+                            if (!phase_barrier(E, sm, W)) return false;
+                        }
+                        const int rbn = tf_rows(n), cw = tf_tile_width(n, rbn, W.count);
+                        const long long units = tf_units(n, rbn, cw);
+                        const long long a = units * W.id / W.count, b = units * (W.id + 1) / W.count;
+                        for (long long u = a; u < b;) {
+                            u = ts_filter_tiles(E, n, rbn, cw, u, b, sm);
+                            ts_filter_merge<PREC>(E, S, n, rbn, cw, u, sm);
+                        }
+                    }
+                } else if (PREC == HHS_PREC_FP64) {
                     nch = chunks_for(n, W, true, E.units_per_cta);
                     const int C = (n + nch - 1) / nch;
                     const int nsb = (n + kEB - 1) / kEB;
@@ -3233,17 +3668,6 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                         ts_unit<PREC>(E, S, n, ib, j0, j1, E.ts_part + (size_t)jc * E.n_max,
                                       nullptr, sm);
                     }
-                } else if (MODE == kModeGrid && E.tq) {
-                    // packed members: written by the parent's kick-reduce phase when it
-                    // ran (the second pass of a fast set), else packed here
-                    if (lvl == top || ld_volatile_i32(&E.counts[lvl - 1].n_slow) == 0) {
-                        pack_ts(E, S, n, W);
-                        if (!phase_barrier(E, sm, W)) return false;
-                    }
-                    const int cw = ts_tile_width(n, W.count);
-                    const long long units = ts_tile_units(n, cw);
-                    ts_sym_tiles(E, n, cw, units * W.id / W.count, units * (W.id + 1) / W.count,
-                                 sm);
                 } else {
                     // only units with a pair j > i: row block rb takes column blocks
                     // cb >= rb * kEB / kCB; each worker takes a contiguous range of that
@@ -3257,7 +3681,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 prof_mark(E, W, t_last, kProfTs, (double)n * (double)(n - 1), sm, lvl);
             }
             if constexpr (MODE == kModeGrid) {
-                split_phase<PREC>(E, S, n, dt, lvl, calc, nch, W, sm);
+                split_phase<PREC, FILTER>(E, S, n, dt, lvl, calc, nch, filtered, lvl == top, W, sm);
             } else {
                 count_phase<PREC>(E, S, n, dt, calc, nch, W, sm);
                 if (!phase_barrier(E, sm, W)) return false;
@@ -3325,8 +3749,8 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 if (!phase_barrier(E, sm, W)) return false;
                 const double ns_d = ns, nf_d = nf;
                 prof_mark(E, W, t_last, kProfKick, ns_d * (ns_d - 1.0) + 2.0 * ns_d * nf_d, sm, lvl);
-                if (grid_tma) kick_reduce_phase<PREC>(E, F, L, nf, ns, dt, kp.ncs, 0, W, sm, kp.nfsb);
-                else kick_reduce_phase<PREC>(E, F, L, nf, ns, dt, nch, C, W, sm);
+                if (grid_tma) kick_reduce_phase<PREC, FILTER>(E, F, L, nf, ns, dt, kp.ncs, 0, W, sm, kp.nfsb);
+                else kick_reduce_phase<PREC, FILTER>(E, F, L, nf, ns, dt, nch, C, W, sm);
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfUpdate, 0.0, sm, lvl);
             }
@@ -3345,10 +3769,9 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
     return true;
 }
 
-template <int PREC>
-__global__ void __launch_bounds__(kEB, 2) k_engine(EParams E) {
-    extern __shared__ __align__(16) unsigned char engine_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
+template <int PREC, bool FILTER>
+__global__ void __launch_bounds__(kEB, 2) k_engine(const __grid_constant__ EParams E) {
+    Smem& sm = cta_smem();
     const Workers W{(int)blockIdx.x, (int)gridDim.x, kModeGrid};
     if (threadIdx.x == 0) {
         sm.bar_k = 0u;  // thread 0 alone uses it
@@ -3363,7 +3786,7 @@ __global__ void __launch_bounds__(kEB, 2) k_engine(EParams E) {
     unsigned long long t_last = 0;
     prof_begin(E, sm);
     prof_mark(E, W, t_last, -1, 0.0, sm);
-    run_hold<PREC, kModeGrid>(E, E.top_level, E.calc_top != 0, W, sm, t_last);
+    run_hold<PREC, kModeGrid, FILTER>(E, E.top_level, E.calc_top != 0, W, sm, t_last);
     prof_end(E, sm);
 }
 
@@ -3374,8 +3797,7 @@ __global__ void __launch_bounds__(kEB, 2) k_engine(EParams E) {
 // all others), written to E.ts_part / rate_acc / tile_counts reinterpreted as FP64
 // ax / ay / az (see engine_kick_accelerations).
 __global__ void __launch_bounds__(kEB, 2) k_engine_accel(EParams E) {
-    extern __shared__ __align__(16) unsigned char engine_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
+    Smem& sm = cta_smem();
     const Workers W{(int)blockIdx.x, (int)gridDim.x, kModeGrid};
     if (threadIdx.x == 0) {
         sm.bar_k = 0u;
@@ -3425,8 +3847,7 @@ __global__ void __launch_bounds__(kEB, 2) k_engine_accel(EParams E) {
 // tiles bulk-copied, one rate per unordered pair, row and column maxima), then converted
 // to timesteps as the split phase does, into P.ts (see engine_timestep_rates).
 __global__ void __launch_bounds__(kEB, 2) k_engine_ts(EParams E) {
-    extern __shared__ __align__(16) unsigned char engine_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
+    Smem& sm = cta_smem();
     const Workers W{(int)blockIdx.x, (int)gridDim.x, kModeGrid};
     if (threadIdx.x == 0) {
         sm.bar_k = 0u;
@@ -3443,7 +3864,7 @@ __global__ void __launch_bounds__(kEB, 2) k_engine_ts(EParams E) {
     if (!grid_barrier(E, sm)) return;
     const int cw = ts_tile_width(n, W.count);
     const long long units = ts_tile_units(n, cw);
-    ts_sym_tiles(E, n, cw, units * W.id / W.count, units * (W.id + 1) / W.count, sm);
+    ts_sym_tiles(E, n, cw, units * W.id / W.count, units * (W.id + 1) / W.count);
     if (!grid_barrier(E, sm)) return;
     for (int i = W.id * kEB + (int)threadIdx.x; i < n; i += W.count * kEB) {
         const float mr = __uint_as_float(E.rate_acc[i]);
@@ -3473,8 +3894,7 @@ __device__ __forceinline__ void kick_smem_init(Smem& sm) {
 __global__ void __launch_bounds__(kEB, 2)
     k_shard_ts_mixed(EParams E, const int32_t* S, int n, long long u_lo, long long u_hi,
                      PeerOut po) {
-    extern __shared__ __align__(16) unsigned char engine_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
+    Smem& sm = cta_smem();
     const long long span = u_hi - u_lo;
     const int u0 = (int)(u_lo + span * blockIdx.x / gridDim.x);
     const int u1 = (int)(u_lo + span * (blockIdx.x + 1) / gridDim.x);
@@ -3496,8 +3916,7 @@ __global__ void k_rates_to_ts(EParams E, const int32_t* S, int n) {
 // in ts_part; then the minimum of each sink of [s_lo, s_hi) to every replica.
 __global__ void __launch_bounds__(kEB, 2)
     k_shard_ts_fp64(EParams E, const int32_t* S, int n, int ib_lo, int ib_hi, int nch) {
-    extern __shared__ __align__(16) unsigned char engine_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
+    Smem& sm = cta_smem();
     const int C = (n + nch - 1) / nch;
     const int units = (ib_hi - ib_lo) * nch;
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
@@ -3537,8 +3956,7 @@ __global__ void k_pack_slow(EParams E, const int32_t* L, int ns, int lvl) {
 __global__ void __launch_bounds__(kEB, 2)
     k_shard_kick_mixed(EParams E, const int32_t* F, int nf, int ns, int lvl, int nch, int C,
                        int ib_lo, int ib_hi) {
-    extern __shared__ __align__(16) unsigned char engine_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
+    Smem& sm = cta_smem();
     kick_smem_init(sm);
     const Workers W{(int)blockIdx.x, (int)gridDim.x, kModeGrid};
     kick_units_grid(E, F, nf, ns, lvl, nch, C, W, sm, ib_lo, ib_hi);
@@ -3549,8 +3967,7 @@ __global__ void __launch_bounds__(kEB, 2)
 __global__ void __launch_bounds__(kEB, 2)
     k_shard_kick_fp64(EParams E, const int32_t* F, const int32_t* L, int nf, int ns, int s_lo,
                       int s_hi) {
-    extern __shared__ __align__(16) unsigned char engine_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(engine_smem);
+    Smem& sm = cta_smem();
     const Workers W{(int)blockIdx.x, (int)gridDim.x, kModeGrid};
     kick_fp64_units(E, F, L, nf, ns, 0.0, nullptr, s_lo, s_hi, nullptr, W, sm);
 }
@@ -3642,8 +4059,7 @@ __device__ __forceinline__ EParams system_params(const BParams& B, int sys, cons
 
 template <int PREC>
 __global__ void __launch_bounds__(kEB, 2) k_batched(BParams B) {
-    extern __shared__ __align__(16) unsigned char batched_smem[];
-    Smem& sm = *reinterpret_cast<Smem*>(batched_smem);
+    Smem& sm = cta_smem();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int cs = (int)cluster.num_blocks();
@@ -3661,7 +4077,7 @@ __global__ void __launch_bounds__(kEB, 2) k_batched(BParams B) {
         const int sys = B.order[idx];
         const EParams E = system_params(B, sys, B.cluster_slots + (size_t)cid * B.cluster_slot_bytes);
         const Workers W{rank, cs, kModeCluster};
-        run_hold<PREC, kModeCluster>(E, 0, E.calc_top != 0, W, sm, t);
+        run_hold<PREC, kModeCluster, false>(E, 0, E.calc_top != 0, W, sm, t);
     }
     // small systems: one CTA per system
     while (true) {
@@ -3673,7 +4089,7 @@ __global__ void __launch_bounds__(kEB, 2) k_batched(BParams B) {
         const int sys = B.order[B.n_big + idx];
         const EParams E = system_params(B, sys, B.cta_slots + (size_t)blockIdx.x * B.cta_slot_bytes);
         const Workers W{0, 1, kModeBlock};
-        run_hold<PREC, kModeBlock>(E, 0, E.calc_top != 0, W, sm, t);
+        run_hold<PREC, kModeBlock, false>(E, 0, E.calc_top != 0, W, sm, t);
     }
 }
 
@@ -3702,6 +4118,8 @@ struct EngineHost {
     double* c_part = nullptr;
     float4* tq = nullptr;
     long long tq_stride = 0;
+    float4* tf = nullptr;
+    unsigned long long* tau_key = nullptr;
     int32_t* trace = nullptr;                 // caller's node-record buffer (4 int32 each)
     unsigned long long* trace_count = nullptr;
     long long trace_cap = 0;
@@ -3710,6 +4128,18 @@ struct EngineHost {
 constexpr size_t kAl = 256;
 inline size_t al(size_t v) { return (v + kAl - 1) & ~(kAl - 1); }
 
+}  // namespace
+
+namespace {
+// the kernels of the device step
+std::array<const void*, 3> engine_kernels() {
+    return {(const void*)k_engine<HHS_PREC_FP64, true>, (const void*)k_engine<HHS_PREC_MIXED, false>,
+            (const void*)k_engine<HHS_PREC_MIXED, true>};
+}
+// Mixed steps filter their timesteps from here on: at 16384 particles the filter saves 1.9 of 4.1
+// ms of timesteps, at 4099 0.04 of 0.41, and its code costs the subtree solver in the same kernel
+// 3% (registers). FP64 steps always do (a full FP64 evaluation takes ten times as long).
+constexpr int kFilterN = 6000;
 }  // namespace
 
 // levels with packed kick sources (deeper levels, if they run grid phases at all, gather)
@@ -3722,7 +4152,8 @@ size_t engine_workspace_bytes(int n_max, int max_levels) {
            al(sizeof(double) * kMaxChunks * 3 * n) + al(sizeof(int) * (n / kEB + 2)) +
            al(sizeof(unsigned) * n) + al(sizeof(unsigned long long) * (n / kEB + 2)) +
            al(sizeof(float4) * 4 * (n / 2 + 1) * (size_t)pk_levels_for(max_levels)) +
-           al(sizeof(double) * kMaxFsb * 3 * n) + al(sizeof(float4) * 5 * (n / 2 + 1));
+           al(sizeof(double) * kMaxFsb * 3 * n) + al(sizeof(float4) * 5 * (n / 2 + 1)) +
+           al(sizeof(float4) * 5 * (n / 2 + 1)) + al(sizeof(unsigned long long) * n);
 }
 
 hhs_status engine_init(hhs_ctx* c, void* base) {
@@ -3742,7 +4173,9 @@ hhs_status engine_init(hhs_ctx* c, void* base) {
     eh->pk = reinterpret_cast<float4*>(p);
     p += al(sizeof(float4) * 4 * (size_t)eh->pk_stride * (size_t)eh->pk_levels);
     eh->c_part = reinterpret_cast<double*>(p); p += al(sizeof(double) * kMaxFsb * 3 * n);
-    eh->tq = reinterpret_cast<float4*>(p);
+    eh->tq = reinterpret_cast<float4*>(p); p += al(sizeof(float4) * 5 * (n / 2 + 1));
+    eh->tf = reinterpret_cast<float4*>(p); p += al(sizeof(float4) * 5 * (n / 2 + 1));
+    eh->tau_key = reinterpret_cast<unsigned long long*>(p);
     eh->tq_stride = (long long)(n / 2 + 1);
     eh->n_max = c->n_max;
     int dev = 0, sms = 0, coop = 0;
@@ -3751,19 +4184,19 @@ hhs_status engine_init(hhs_ctx* c, void* base) {
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     if (!coop) { delete eh; return HHS_ERR_CUDA; }
     int b0 = 0, b1 = 0;
-    HHS_CUDA_TRY(cudaFuncSetAttribute(k_engine<HHS_PREC_FP64>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEngineSmem));
-    HHS_CUDA_TRY(cudaFuncSetAttribute(k_engine<HHS_PREC_MIXED>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEngineSmem));
+    for (const void* k : engine_kernels())
+        HHS_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)kEngineSmem));
     HHS_CUDA_TRY(cudaFuncSetAttribute(k_engine_accel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kEngineSmem));
     HHS_CUDA_TRY(cudaFuncSetAttribute(k_engine_ts, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kEngineSmem));
     // clusters of 16 CTAs (beyond the portable 8) for the subtree solver, where allowed
-    if (cudaFuncSetAttribute(k_engine<HHS_PREC_FP64>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_engine<HHS_PREC_MIXED>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess ||
+    bool big = true;
+    for (const void* k : engine_kernels())
+        big = big && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                         cudaSuccess;
+    if (!big ||
         cudaFuncSetAttribute(k_engine_accel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_engine_ts, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
@@ -3777,10 +4210,14 @@ hhs_status engine_init(hhs_ctx* c, void* base) {
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEngineSmem));
     HHS_CUDA_TRY(cudaFuncSetAttribute(k_shard_kick_fp64,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEngineSmem));
-    HHS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_engine<HHS_PREC_FP64>, kEB,
-                                                               kEngineSmem));
-    HHS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_engine<HHS_PREC_MIXED>, kEB,
-                                                               kEngineSmem));
+    HHS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_engine<HHS_PREC_FP64, true>,
+                                                               kEB, kEngineSmem));
+    HHS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_engine<HHS_PREC_MIXED, false>,
+                                                               kEB, kEngineSmem));
+    int b2 = 0;  // both mixed kernels run with one grid
+    HHS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k_engine<HHS_PREC_MIXED, true>,
+                                                               kEB, kEngineSmem));
+    b1 = b1 < b2 ? b1 : b2;
     eh->sms = sms;
     eh->occ[0] = b0;
     eh->occ[1] = b1;
@@ -3835,9 +4272,13 @@ hhs_status engine_set_tuning(hhs_ctx* c, const hhs_tuning& t) {
             at[0].val.clusterDim.z = 1;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            const cudaError_t e =
-                k == 0 ? cudaOccupancyMaxActiveClusters(&nc, (void*)k_engine<HHS_PREC_FP64>, &cfg)
-                       : cudaOccupancyMaxActiveClusters(&nc, (void*)k_engine<HHS_PREC_MIXED>, &cfg);
+            cudaError_t e = cudaOccupancyMaxActiveClusters(
+                &nc, k == 0 ? (void*)k_engine<HHS_PREC_FP64, true> : (void*)k_engine<HHS_PREC_MIXED, false>,
+                &cfg);
+            int nc2 = nc;
+            if (e == cudaSuccess && k == 1)
+                e = cudaOccupancyMaxActiveClusters(&nc2, (void*)k_engine<HHS_PREC_MIXED, true>, &cfg);
+            nc = nc < nc2 ? nc : nc2;
             if (e != cudaSuccess || nc <= 0) return HHS_ERR_CUDA;
             const int gc = nc * t.cluster_size;
             g = (g < gc ? g : gc) / t.cluster_size * t.cluster_size;
@@ -3918,6 +4359,8 @@ hhs_status engine_reset_barrier(hhs_ctx* c, cudaStream_t stream) {
     if (!eh) return HHS_ERR_INVALID_ARG;
     HHS_CUDA_TRY(cudaMemsetAsync(eh->st, 0, 2 * sizeof(unsigned), stream));
     HHS_CUDA_TRY(cudaMemsetAsync(eh->rate_acc, 0, sizeof(unsigned) * (size_t)eh->n_max, stream));
+    HHS_CUDA_TRY(cudaMemsetAsync(eh->tau_key, 0, sizeof(unsigned long long) * (size_t)eh->n_max,
+                                 stream));
     return HHS_OK;
 }
 
@@ -3955,6 +4398,10 @@ EParams engine_params(hhs_ctx* c, EngineHost* eh, const SoA& P, int n, double dt
     E.c_part = eh->c_part;
     E.tq = eh->tq;
     E.tq_stride = eh->tq_stride;
+    E.tf = eh->tf;
+    E.tau_key = eh->tau_key;
+    // the bounds are guessed from timesteps that this launch computed
+    E.filter = calc_ts && E.eta <= 1.0 ? 1 : 0;
     E.tile_counts = eh->tile_counts;
     E.tile_status = eh->tile_status;
     E.rate_acc = eh->rate_acc;
@@ -3993,7 +4440,7 @@ cudaError_t engine_launch(EngineHost* eh, int pi, K kernel, const EParams& E, cu
     }
     // the grid barrier counts this launch's arrivals from zero; look-back words of earlier
     // launches must not look ready
-    cudaError_t e = cudaMemsetAsync(&eh->st->bar_count, 0, sizeof(unsigned), stream);
+    cudaError_t e = cudaMemsetAsync(&eh->st->bar_count, 0, 2 * sizeof(unsigned), stream);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(eh->tile_status, 0,
                             sizeof(unsigned long long) * (size_t)(eh->n_max / kEB + 2), stream);
@@ -4011,8 +4458,10 @@ hhs_status engine_hold_step(hhs_ctx* c, const SoA& P, int n, double dt, bool cal
     EParams E = engine_params(c, eh, P, n, dt, calc_ts, profile, top_level);
     const int pi = prec == HHS_PREC_FP64 ? 0 : 1;
     E.prec_mixed = pi;
-    const cudaError_t e = pi == 0 ? engine_launch(eh, 0, k_engine<HHS_PREC_FP64>, E, stream)
-                                  : engine_launch(eh, 1, k_engine<HHS_PREC_MIXED>, E, stream);
+    const cudaError_t e = pi == 0 ? engine_launch(eh, 0, k_engine<HHS_PREC_FP64, true>, E, stream)
+                          : n < kFilterN
+                              ? engine_launch(eh, 1, k_engine<HHS_PREC_MIXED, false>, E, stream)
+                              : engine_launch(eh, 1, k_engine<HHS_PREC_MIXED, true>, E, stream);
     hhs_count_launch();
     if (e != cudaSuccess) return hhs_from_cuda(e);
     return HHS_OK;
@@ -4335,6 +4784,9 @@ extern "C" hhs_status hhs_hold_batched(hhs_batch* b, hhs_particle_system* sys, d
     E.ts_part = E.k_part = E.c_part = nullptr;
     E.tq = nullptr;
     E.tq_stride = 0;
+    E.tf = nullptr;
+    E.tau_key = nullptr;
+    E.filter = 0;
     E.tile_counts = nullptr;
     E.tile_status = nullptr;
     E.rate_acc = nullptr;
