@@ -14,7 +14,6 @@ using namespace hhs;
 
 namespace {
 
-constexpr int kTsBlock = 128;
 constexpr int kKickBlock = 128;
 constexpr double kHuge = 1.e30;  // src/timestep.cuh:4
 
@@ -36,96 +35,214 @@ __device__ __forceinline__ void peer_store_v(const PeerOut& po, int g, double vx
     __threadfence_system();
 }
 
-// ---------------------------------------------------------------- timesteps, FP64
-__global__ void __launch_bounds__(kTsBlock)
-    k_timesteps_fp64(SoA P, const int32_t* __restrict__ list, int n, double eta,
-                     double eta_s2, PeerOut po) {
-    __shared__ double sx[kTsBlock], sy[kTsBlock], sz[kTsBlock];
-    __shared__ double svx[kTsBlock], svy[kTsBlock], svz[kTsBlock], sm[kTsBlock];
-    const int i = po.lo + blockIdx.x * kTsBlock + threadIdx.x;
-    const bool active = i < (po.hi < 0 ? n : po.hi);
-    const int gi = active ? list_at(list, i) : 0;
-    double xi = 0, yi = 0, zi = 0, vxi = 0, vyi = 0, vzi = 0, mi = 0;
-    if (active) {
-        xi = P.x[gi]; yi = P.y[gi]; zi = P.z[gi];
-        vxi = P.vx[gi]; vyi = P.vy[gi]; vzi = P.vz[gi];
-        mi = P.m[gi];
-    }
-    double minval = kHuge;
-    for (int jt = 0; jt < n; jt += kTsBlock) {
-        const int j = jt + threadIdx.x;
-        if (j < n) {
-            const int gj = list_at(list, j);
-            sx[threadIdx.x] = P.x[gj]; sy[threadIdx.x] = P.y[gj]; sz[threadIdx.x] = P.z[gj];
-            svx[threadIdx.x] = P.vx[gj]; svy[threadIdx.x] = P.vy[gj];
-            svz[threadIdx.x] = P.vz[gj]; sm[threadIdx.x] = P.m[gj];
-        }
-        __syncthreads();
-        if (active) {
-            const int jn = min(kTsBlock, n - jt);
-            for (int jl = 0; jl < jn; jl++) {
-                if (jt + jl == i) continue;
-                ts_pair_fp64(f64_sub(xi, sx[jl]), f64_sub(yi, sy[jl]), f64_sub(zi, sz[jl]),
-                             f64_sub(vxi, svx[jl]), f64_sub(vyi, svy[jl]), f64_sub(vzi, svz[jl]), mi,
-                             sm[jl], eta, eta_s2, minval);
-            }
-        }
-        __syncthreads();
-    }
-    if (active) {
-        P.ts[gi] = minval;
-        peer_store_ts(po, gi, minval);
-    }
+// ---------------------------------------------------------------- timesteps
+// A CTA takes T rows (particles) and passes over all n columns, 512 at a time, two a thread in
+// registers, with the pair test of the device step's filtered timestep (hhs_engine.cu): a pair
+// below a row's best rate so far is left out by 9 packed FP32 operations for two pairs, and the
+// few that pass are listed and evaluated exactly, in either precision, some dozens at a time.
+// Each row starts from its exact rates over the first 32 columns. The result is the maximum
+// over all pairs, as if every one had been evaluated.
+//
+// The test here is for the row alone, with its rate T = 0.99 best: a pair may be left out if
+//     A >= kappa B + C (p_i + p_j) and B >= D (p_i + p_j),  p = |m|^(2/3),
+// A = |x_i - x_j|^2, B = |v_i - v_j|^2, C = (2 / (eta beta T)^2)^(2/3), D = (1 / (2 (1 - alpha)
+// T C))^2: C (p_i + p_j) is at least the `a` and D (p_i + p_j) at least the `b` of the pair's
+// mass sum there, since (m_i + m_j)^(2/3) <= p_i + p_j.
+//
+// Measured, one call: 2051 particles in FP64 1384 -> 23 us, 16384 mixed 1652 -> 261 us. What
+// bounds it: the latency of a row's test (a chain of six packed operations, its shared-memory
+// reads and a branch, hidden by eight warps per scheduler at most), and below about 4000
+// particles that of a tile's loads and listed pairs.
+constexpr int kTsThreads = 256;
+constexpr int kTsCols = 2 * kTsThreads;  // columns of a tile
+constexpr int kTsSeed = 32;              // columns that every row evaluates first
+constexpr int kTsCap = 2048;             // pairs listed at a time
+constexpr unsigned kTsBatch = 64;        // listed pairs that are worth evaluating together
+constexpr int kTsMaxRows = 32;
+constexpr float kTsAlpha = 0.9f;
+constexpr float kTsAll = 1.0e38f;
+
+struct __align__(16) TsRowTest {  // -2 x, -2 v, -kappa, -C, -D, each in both lanes; pass: v <= c1 or w < c2
+    float2 x, y, z, vx, vy, vz, nk, nC, nD;
+    float c1, c2;
+};
+
+struct TsArgs {
+    double eta, eta_s2;
+    float inv_eta_s2, inv_eta;
+};
+
+struct TsState {
+    double x, y, z, vx, vy, vz, m;
+};
+
+__device__ __forceinline__ TsState ts_load(const SoA& P, int g) {
+    return TsState{P.x[g], P.y[g], P.z[g], P.vx[g], P.vy[g], P.vz[g], P.m[g]};
 }
 
-// ---------------------------------------------------------------- timesteps, mixed
-__global__ void __launch_bounds__(kTsBlock)
-    k_timesteps_mixed(SoA P, const int32_t* __restrict__ list, int n, float inv_eta_s2,
-                      float inv_eta, PeerOut po) {
-    __shared__ float4 sA[kTsBlock];  // xh, yh, zh, m
-    __shared__ float4 sB[kTsBlock];  // xl, yl, zl, -
-    __shared__ float4 sV[kTsBlock];  // vx, vy, vz, -
-    const int i = po.lo + blockIdx.x * kTsBlock + threadIdx.x;
-    const bool active = i < (po.hi < 0 ? n : po.hi);
-    const int gi = active ? list_at(list, i) : 0;
-    DS xi{0, 0}, yi{0, 0}, zi{0, 0};
-    float vxi = 0, vyi = 0, vzi = 0, mi = 0;
-    if (active) {
-        xi = ds_split(P.x[gi]); yi = ds_split(P.y[gi]); zi = ds_split(P.z[gi]);
-        vxi = (float)P.vx[gi]; vyi = (float)P.vy[gi]; vzi = (float)P.vz[gi];
-        mi = (float)P.m[gi];
+// the pair's rate as FP32 bits (mixed) or the complement of its timescale's bits (FP64): the
+// largest key is the timestep; 0 for none
+template <int PREC>
+__device__ __forceinline__ unsigned long long ts_key(const TsState& a, const TsState& b,
+                                                     const TsArgs& A) {
+    if constexpr (PREC == HHS_PREC_FP64) {
+        double t = kHuge;
+        ts_pair_fp64(f64_sub(a.x, b.x), f64_sub(a.y, b.y), f64_sub(a.z, b.z), f64_sub(a.vx, b.vx),
+                     f64_sub(a.vy, b.vy), f64_sub(a.vz, b.vz), a.m, b.m, A.eta, A.eta_s2, t);
+        return t < kHuge ? ~(unsigned long long)__double_as_longlong(t) : 0ull;
+    } else {
+        const DS ax = ds_split(a.x), ay = ds_split(a.y), az = ds_split(a.z);
+        const DS bx = ds_split(b.x), by = ds_split(b.y), bz = ds_split(b.z);
+        const float r = ts_pair_rate_mixed(
+            ds_diff(ax.hi, ax.lo, bx.hi, bx.lo), ds_diff(ay.hi, ay.lo, by.hi, by.lo),
+            ds_diff(az.hi, az.lo, bz.hi, bz.lo), (float)a.vx - (float)b.vx,
+            (float)a.vy - (float)b.vy, (float)a.vz - (float)b.vz, (float)a.m + (float)b.m,
+            A.inv_eta_s2, A.inv_eta);
+        return r > 0.0f ? (unsigned long long)__float_as_uint(r) : 0ull;
     }
-    float maxrate = 0.0f;
-    for (int jt = 0; jt < n; jt += kTsBlock) {
-        const int j = jt + threadIdx.x;
-        if (j < n) {
-            const int gj = list_at(list, j);
-            const DS a = ds_split(P.x[gj]), b = ds_split(P.y[gj]), c = ds_split(P.z[gj]);
-            sA[threadIdx.x] = make_float4(a.hi, b.hi, c.hi, (float)P.m[gj]);
-            sB[threadIdx.x] = make_float4(a.lo, b.lo, c.lo, 0.0f);
-            sV[threadIdx.x] =
-                make_float4((float)P.vx[gj], (float)P.vy[gj], (float)P.vz[gj], 0.0f);
+}
+template <int PREC>
+__device__ __forceinline__ double ts_of_key(unsigned long long key) {
+    if (key == 0ull) return kHuge;
+    if (PREC == HHS_PREC_FP64) return __longlong_as_double((long long)~key);
+    const double t = 1.0 / (double)__uint_as_float((unsigned)key);
+    return t < kHuge ? t : kHuge;
+}
+
+template <int PREC>
+__device__ __forceinline__ TsRowTest ts_row_test(const TsState& q, unsigned long long key,
+                                                 const TsArgs& A) {
+    TsRowTest r;
+    const double rate = 1.0 / ts_of_key<PREC>(key), r2 = q.x * q.x + q.y * q.y + q.z * q.z,
+                 v2 = q.vx * q.vx + q.vy * q.vy + q.vz * q.vz;
+    const float T = 0.99f * (float)rate, eta = (float)A.eta;
+    const float e = 1.0f / eta + 0.5f, beta = 1.0f - 0.75f * kTsAlpha / e;
+    const float k = e / (kTsAlpha * T), f = eta * beta * T, c = cbrtf(2.01f / (f * f));
+    const float kappa = 1.01f * k * k, C = 1.02f * c * c;
+    const float h = 0.5f / ((1.0f - kTsAlpha) * T * C), D = 1.02f * h * h;
+    const float pm = cbrtf((float)fabs(q.m)), p = 1.01f * pm * pm;
+    const float W = (float)(r2 * (1.0 - 4e-6)), U = (float)(v2 * (1.0 + 4e-6));
+    // without a usable rate (or for eta beyond the test's range) every pair passes
+    const bool ok = A.eta <= 1.0 && rate > 1e-12 && rate < 1e12 && r2 < 1e24 && v2 < 1e24 &&
+                    kappa < 1e24f && C * p < 1e24f && D * p < 1e24f;
+    r.x = f2dup(ok ? -2.0f * (float)q.x : 0.0f);
+    r.y = f2dup(ok ? -2.0f * (float)q.y : 0.0f);
+    r.z = f2dup(ok ? -2.0f * (float)q.z : 0.0f);
+    r.vx = f2dup(ok ? -2.0f * (float)q.vx : 0.0f);
+    r.vy = f2dup(ok ? -2.0f * (float)q.vy : 0.0f);
+    r.vz = f2dup(ok ? -2.0f * (float)q.vz : 0.0f);
+    r.nk = f2dup(ok ? -kappa : 0.0f);
+    r.nC = f2dup(ok ? -C : 0.0f);
+    r.nD = f2dup(ok ? -D : 0.0f);
+    const float a = C * p + 1e-30f;
+    r.c1 = ok ? (a - W + kappa * U) + 2e-6f * (a + W + kappa * U) : 3e38f;
+    r.c2 = ok ? D * p + 4e-5f * U + 1e-30f - U : 3e38f;
+    return r;
+}
+
+template <int PREC>
+__global__ void __launch_bounds__(kTsThreads, 4)
+    k_timesteps(SoA P, const int32_t* __restrict__ list, int n, int T, TsArgs A, PeerOut po) {
+    __shared__ TsState row[kTsMaxRows];
+    __shared__ TsRowTest test[kTsMaxRows];
+    __shared__ unsigned long long best[kTsMaxRows];
+    __shared__ int2 hit[kTsCap];  // (row, column)
+    __shared__ unsigned s_cnt;
+    const int tid = threadIdx.x;
+    const int hi = po.hi < 0 ? n : po.hi;
+    const int i0 = po.lo + blockIdx.x * T, nrow = min(T, hi - i0);
+    if (tid < nrow) row[tid] = ts_load(P, list_at(list, i0 + tid));
+    if (tid < kTsMaxRows) best[tid] = 0ull;
+    if (tid == 0) s_cnt = 0u;
+    __syncthreads();
+    for (int k = tid; k < nrow * kTsSeed; k += kTsThreads) {
+        const int r = k / kTsSeed, j = k % kTsSeed;
+        if (j < n && j != i0 + r) {
+            const unsigned long long q = ts_key<PREC>(row[r], ts_load(P, list_at(list, j)), A);
+            if (q > best[r]) atomicMax(&best[r], q);
         }
-        __syncthreads();
-        if (active) {
-            const int jn = min(kTsBlock, n - jt);
-            for (int jl = 0; jl < jn; jl++) {
-                if (jt + jl == i) continue;
-                const float4 A = sA[jl], B = sB[jl], V = sV[jl];
-                const float rate = ts_pair_rate_mixed(
-                    ds_diff(xi.hi, xi.lo, A.x, B.x), ds_diff(yi.hi, yi.lo, A.y, B.y),
-                    ds_diff(zi.hi, zi.lo, A.z, B.z), vxi - V.x, vyi - V.y, vzi - V.z, mi + A.w,
-                    inv_eta_s2, inv_eta);
-                maxrate = fmaxf(maxrate, rate);
+    }
+    __syncthreads();
+    if (tid < nrow) test[tid] = ts_row_test<PREC>(row[tid], best[tid], A);
+    __syncthreads();
+    unsigned held = 0u;
+    for (int t0 = 0; t0 < n; t0 += kTsCols) {
+        const int j0 = t0 + 2 * tid;
+        float2 X, Y, Z, VX, VY, VZ, W, U, p;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const TsState q = j0 + c < n ? ts_load(P, list_at(list, j0 + c))
+                                         : TsState{0, 0, 0, 0, 0, 0, 0};
+            const double r2 = q.x * q.x + q.y * q.y + q.z * q.z,
+                         v2 = q.vx * q.vx + q.vy * q.vy + q.vz * q.vz;
+            const float pm = cbrtf((float)fabs(q.m)), pc = 1.01f * pm * pm;
+            const bool ok = r2 < 1e24 && v2 < 1e24 && pc < 1e20f;  // else it passes every test
+            auto put = [&](float2& v, float f) {
+                if (c) v.y = f;
+                else v.x = f;
+            };
+            put(X, ok ? (float)q.x : 0.0f);
+            put(Y, ok ? (float)q.y : 0.0f);
+            put(Z, ok ? (float)q.z : 0.0f);
+            put(VX, ok ? (float)q.vx : 0.0f);
+            put(VY, ok ? (float)q.vy : 0.0f);
+            put(VZ, ok ? (float)q.vz : 0.0f);
+            put(p, ok ? pc : 0.0f);
+            put(W, ok ? (float)(r2 * (1.0 - 4e-6)) : -kTsAll);
+            put(U, ok ? (float)(v2 * (1.0 + 4e-6)) : 0.0f);
+        }
+        for (int r = 0; r < nrow; r++) {
+            __syncwarp();  // lanes that listed pairs rejoin the others here
+            const TsRowTest t = test[r];
+            float2 w = __ffma2_rn(t.vx, VX, U), v = __ffma2_rn(t.x, X, W);
+            w = __ffma2_rn(t.vy, VY, w);
+            v = __ffma2_rn(t.y, Y, v);
+            w = __ffma2_rn(t.vz, VZ, w);
+            v = __ffma2_rn(t.z, Z, v);
+            v = __ffma2_rn(t.nk, w, v);
+            v = __ffma2_rn(t.nC, p, v);
+            w = __ffma2_rn(t.nD, p, w);
+            if (fminf(v.x, v.y) <= t.c1 || fminf(w.x, w.y) < t.c2) {
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const float vc = c ? v.y : v.x, wc = c ? w.y : w.x;
+                    if ((vc <= t.c1 || wc < t.c2) && j0 + c < n && j0 + c != i0 + r) {
+                        const unsigned k = atomicAdd(&s_cnt, 1u);
+                        if (k < kTsCap) hit[k] = make_int2(r, j0 + c);
+                    }
+                }
             }
         }
         __syncthreads();
+        const unsigned cnt = s_cnt;
+        __syncthreads();  // every thread has the count
+        if (cnt < kTsBatch && t0 + kTsCols < n) {
+            held = cnt;
+            continue;
+        }
+        // the listed pairs; if the list overflowed, those of earlier tiles and every pair of
+        // this one
+        const bool all = cnt > kTsCap;
+        const int listed = (int)(all ? held : cnt), total = listed + (all ? nrow * kTsCols : 0);
+        for (int k = tid; k < total; k += kTsThreads) {
+            const int2 h = k < listed ? hit[k]
+                                      : make_int2((k - listed) / kTsCols, t0 + (k - listed) % kTsCols);
+            if (h.y >= n || h.y == i0 + h.x) continue;
+            const unsigned long long key =
+                ts_key<PREC>(row[h.x], ts_load(P, list_at(list, h.y)), A);
+            if (key > *(volatile unsigned long long*)&best[h.x]) atomicMax(&best[h.x], key);
+        }
+        __syncthreads();
+        if (tid == 0) s_cnt = 0u;
+        if (tid < nrow) test[tid] = ts_row_test<PREC>(row[tid], best[tid], A);
+        __syncthreads();
+        held = 0u;
     }
-    if (active) {
-        double t = 1.0 / (double)maxrate;
-        t = (t < kHuge) ? t : kHuge;
-        P.ts[gi] = t;
-        peer_store_ts(po, gi, t);
+    if (tid < nrow) {
+        const int g = list_at(list, i0 + tid);
+        const double t = ts_of_key<PREC>(best[tid]);
+        P.ts[g] = t;
+        peer_store_ts(po, g, t);
     }
 }
 
@@ -292,48 +409,94 @@ __global__ void __launch_bounds__(kK64Threads, 2)
     v[i] = f64_add(v[i], f64_mul(a, dtfac));
 }
 
-__global__ void __launch_bounds__(kKickBlock)
+// Mixed: a CTA takes 32 sinks, one a lane, and each of its 8 warps an eighth of the sources, 32
+// at a time, converted to double-single pairs in the warp's own shared memory (no CTA barrier
+// until the end). Two sources are evaluated at once in f32x2 arithmetic, each pair term as
+// before (1/d from rsqrtf with one Newton step) into Kahan-compensated FP32 sums, one for the
+// even and one for the odd sources of each warp; these are added in FP64 in a fixed order.
+// Measured: kick_slow of 10923 particles 926 -> 209 us (one thread a sink before: 86 CTAs, every
+// thread waiting for its own chain of compensated additions). The FMA pipe bounds it: 34 packed
+// operations for two pairs, 12 of them the compensated sums.
+__device__ __forceinline__ void kahan_add2(float2& s, float2& c, float2 t) {
+    const float2 m1 = make_float2(-1.0f, -1.0f);
+    const float2 y = __ffma2_rn(c, m1, t);
+    const float2 u = __fadd2_rn(s, y);
+    c = __ffma2_rn(y, m1, __ffma2_rn(s, m1, u));
+    s = u;
+}
+
+constexpr int kPmWarps = 8;
+__global__ void __launch_bounds__(32 * kPmWarps, 3)
     k_kick_pair_mixed(SoA K, double* __restrict__ ax_out, double* __restrict__ ay_out,
                       double* __restrict__ az_out, SoA S, int n, int m, double dtfac) {
-    __shared__ float4 sA[kKickBlock], sB[kKickBlock];
-    const int i = blockIdx.x * kKickBlock + threadIdx.x;
-    const bool active = i < n;
+    // source pairs: (x hi), (y hi) | (z hi), (mass) | (x lo), (y lo) | (z lo)
+    __shared__ float4 src[kPmWarps][16][4];
+    __shared__ double sum[kPmWarps][3][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     DS xi{0, 0}, yi{0, 0}, zi{0, 0};
-    if (active) { xi = ds_split(K.x[i]); yi = ds_split(K.y[i]); zi = ds_split(K.z[i]); }
-    float acc[3] = {0, 0, 0}, cmp[3] = {0, 0, 0};
-    for (int jt = 0; jt < m; jt += kKickBlock) {
-        const int j = jt + threadIdx.x;
-        if (j < m) {
-            const DS a = ds_split(S.x[j]), b = ds_split(S.y[j]), c = ds_split(S.z[j]);
-            sA[threadIdx.x] = make_float4(a.hi, b.hi, c.hi, (float)S.m[j]);
-            sB[threadIdx.x] = make_float4(a.lo, b.lo, c.lo, 0.0f);
+    if (i < n) { xi = ds_split(K.x[i]); yi = ds_split(K.y[i]); zi = ds_split(K.z[i]); }
+    const float2 nxh = f2dup(-xi.hi), nyh = f2dup(-yi.hi), nzh = f2dup(-zi.hi), nxl = f2dup(-xi.lo),
+                 nyl = f2dup(-yi.lo), nzl = f2dup(-zi.lo);
+    float2 acc[3], cmp[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) acc[k] = cmp[k] = make_float2(0.0f, 0.0f);
+    const int j1 = (int)((long long)m * (warp + 1) / kPmWarps);
+    int j0 = (int)((long long)m * warp / kPmWarps);
+    double sx = 0.0, sy = 0.0, sz = 0.0, sm = 0.0;
+    auto load = [&](int j) {
+        const bool in = j < j1;
+        sx = in ? S.x[j] : 0.0; sy = in ? S.y[j] : 0.0; sz = in ? S.z[j] : 0.0;
+        sm = in ? S.m[j] : 0.0;
+    };
+    load(j0 + lane);
+    for (; j0 < j1; j0 += 32) {
+        __syncwarp();  // the previous sources are read
+        {
+            const DS a = ds_split(sx), b = ds_split(sy), c = ds_split(sz);
+            float* q = reinterpret_cast<float*>(src[warp][lane >> 1]) + (lane & 1);
+            q[0] = a.hi; q[2] = b.hi; q[4] = c.hi; q[6] = (float)sm;
+            q[8] = a.lo; q[10] = b.lo; q[12] = c.lo;
         }
-        __syncthreads();
-        if (active) {
-            const int jn = min(kKickBlock, m - jt);
-            for (int jl = 0; jl < jn; jl++) {
-                const float4 A = sA[jl], B = sB[jl];
-                const float dx = ds_diff(A.x, B.x, xi.hi, xi.lo);
-                const float dy = ds_diff(A.y, B.y, yi.hi, yi.lo);
-                const float dz = ds_diff(A.z, B.z, zi.hi, zi.lo);
-                const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                if (d2 == 0.0f) continue;
-                const float ri = rsqrt_nr(d2);
-                const float mr3 = A.w * ri * ri * ri;
-                kahan_add(acc[0], cmp[0], dx * mr3);
-                kahan_add(acc[1], cmp[1], dy * mr3);
-                kahan_add(acc[2], cmp[2], dz * mr3);
-            }
+        __syncwarp();
+        load(j0 + 32 + lane);  // on its way while these are evaluated
+        const int np = min(32, j1 - j0) + 1 >> 1;
+#pragma unroll 2
+        for (int p = 0; p < np; p++) {
+            const float4 Q0 = src[warp][p][0], Q1 = src[warp][p][1], Q2 = src[warp][p][2];
+            const float2 zl = *reinterpret_cast<const float2*>(&src[warp][p][3]);
+            const float2 dx = __fadd2_rn(__fadd2_rn(make_float2(Q0.x, Q0.y), nxh),
+                                         __fadd2_rn(make_float2(Q2.x, Q2.y), nxl));
+            const float2 dy = __fadd2_rn(__fadd2_rn(make_float2(Q0.z, Q0.w), nyh),
+                                         __fadd2_rn(make_float2(Q2.z, Q2.w), nyl));
+            const float2 dz = __fadd2_rn(__fadd2_rn(make_float2(Q1.x, Q1.y), nzh),
+                                         __fadd2_rn(zl, nzl));
+            float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+            // a particle and itself: no term
+            const float2 w = make_float2(d2.x == 0.0f ? 0.0f : Q1.z, d2.y == 0.0f ? 0.0f : Q1.w);
+            d2.x = d2.x == 0.0f ? 1.0f : d2.x;
+            d2.y = d2.y == 0.0f ? 1.0f : d2.y;
+            const float2 ri = rsqrt_nr2(d2);
+            const float2 mr3 = __fmul2_rn(__fmul2_rn(__fmul2_rn(w, ri), ri), ri);
+            kahan_add2(acc[0], cmp[0], __fmul2_rn(dx, mr3));
+            kahan_add2(acc[1], cmp[1], __fmul2_rn(dy, mr3));
+            kahan_add2(acc[2], cmp[2], __fmul2_rn(dz, mr3));
         }
-        __syncthreads();
     }
-    if (!active) return;
-    const double a0 = (double)acc[0] - cmp[0], a1 = (double)acc[1] - cmp[1],
-                 a2 = (double)acc[2] - cmp[2];
-    if (ax_out) { ax_out[i] = a0; ay_out[i] = a1; az_out[i] = a2; }
-    K.vx[i] += a0 * dtfac;
-    K.vy[i] += a1 * dtfac;
-    K.vz[i] += a2 * dtfac;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        sum[warp][k][lane] = ((double)acc[k].x - (double)cmp[k].x) +
+                             ((double)acc[k].y - (double)cmp[k].y);
+    __syncthreads();
+    if (warp < 3 && i < n) {  // component `warp` of sink i
+        double a = 0.0;
+#pragma unroll
+        for (int w = 0; w < kPmWarps; w++) a += sum[w][warp][lane];
+        double* out = warp == 0 ? ax_out : (warp == 1 ? ay_out : az_out);
+        double* v = warp == 0 ? K.vx : (warp == 1 ? K.vy : K.vz);
+        if (out) out[i] = a;
+        v[i] += a * dtfac;
+    }
 }
 
 // ---------------------------------------------------------------- drift / gathers
@@ -405,12 +568,14 @@ hhs_status launch_timesteps(const SoA& P, const int32_t* list, int n, double eta
     if (hi > n || po.lo > hi) return HHS_ERR_INVALID_ARG;
     if (hi == po.lo) return HHS_OK;  // an empty shard
     const double eta_s2 = eta / 1.41421356237309504880;  // eta / M_SQRT2
-    const int grid = grid_for(hi - po.lo, kTsBlock);
+    const TsArgs A{eta, eta_s2, (float)(1.0 / eta_s2), (float)(1.0 / eta)};
+    // rows of a CTA: the rows share the columns' conversion, but every SM should have its four
+    // CTAs (16384 particles: 261 us with 32 rows, 363 with 64; 32768: 823 with 32, 992 with 64)
+    const int rows = hi - po.lo, T = rows <= 32 * 148 ? 8 : (rows <= 64 * 148 ? 16 : kTsMaxRows);
     if (prec == HHS_PREC_FP64)
-        k_timesteps_fp64<<<grid, kTsBlock, 0, stream>>>(P, list, n, eta, eta_s2, po);
+        k_timesteps<HHS_PREC_FP64><<<grid_for(rows, T), kTsThreads, 0, stream>>>(P, list, n, T, A, po);
     else
-        k_timesteps_mixed<<<grid, kTsBlock, 0, stream>>>(P, list, n, (float)(1.0 / eta_s2),
-                                                         (float)(1.0 / eta), po);
+        k_timesteps<HHS_PREC_MIXED><<<grid_for(rows, T), kTsThreads, 0, stream>>>(P, list, n, T, A, po);
     HHS_LAUNCH_CHECK();
     return HHS_OK;
 }
@@ -448,7 +613,7 @@ hhs_status launch_kick_pair(const SoA& sink, double* ax, double* ay, double* az,
         k_kick_pair_fp64<<<grid_for(n_sink, kK64Pairs >> cs), kK64Threads, bytes, stream>>>(
             sink, ax, ay, az, src, n_sink, n_src, dtfac, cs);
     } else
-        k_kick_pair_mixed<<<grid_for(n_sink, kKickBlock), kKickBlock, 0, stream>>>(
+        k_kick_pair_mixed<<<grid_for(n_sink, 32), 32 * kPmWarps, 0, stream>>>(
             sink, ax, ay, az, src, n_sink, n_src, dtfac);
     HHS_LAUNCH_CHECK();
     return HHS_OK;
