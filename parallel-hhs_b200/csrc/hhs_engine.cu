@@ -55,7 +55,6 @@ constexpr int kTW = 256;          // widest column tile of the packed grid times
 constexpr int kTfCap = 2048;      // pairs that a filtered timestep lists at a time
 constexpr int kMaxFsb = 64;       // fast super-blocks of that kick (column-partial slots)
 constexpr int kMaxChunks = 32;    // source chunks per node (partial-sum slots)
-constexpr int kK64Pairs = 2048;   // pair terms per stage of the FP64 kick
 constexpr int kMaxLevels = 64;    // per-level state is kept in 64-bit masks
 constexpr unsigned long long kBarrierTimeoutNs = 60ull * 1000000000ull;
 
@@ -125,6 +124,9 @@ struct EParams {
 // most kMid particles with its whole subtree lives in shared memory.
 constexpr int kMid = 640;
 constexpr int kMidW = kMid / 32;
+// In FP64 the few SMs of a cluster are throughput bound (a node of 567 members takes 77 us on a
+// cluster of 4, 25 on the grid; one of 241 41 us more): larger nodes stay on the grid.
+constexpr int kMidFp64 = 96;
 struct __align__(16) MidState {
     double x[kMid], y[kMid], z[kMid], vx[kMid], vy[kMid], vz[kMid], m[kMid], ts[kMid];
     float4 A[kMid], B[kMid], V[kMid];     // mixed: position hi + mass, position lo, velocity
@@ -207,7 +209,7 @@ struct __align__(16) Smem {
             int2 hit[kTfCap];                                     // passing pairs
         } tf;
         struct { float4 P0[kEB], P1[kEB], P2[kEB]; float2 M[kEB]; } kx;  // packed kick tiles
-        Kick64Smem<kK64Pairs> k64;                              // FP64 kick terms
+        Kick64Smem k64;                                         // FP64 kick terms
         struct {                                                  // tiny-subtree state
             double x[32], y[32], z[32], vx[32], vy[32], vz[32], m[32], ts[32];
             float4 A[32], B[32], V[32];
@@ -1162,15 +1164,14 @@ __device__ __forceinline__ double4* pk64_level(const EParams& E, int lvl) {
     return reinterpret_cast<double4*>(E.pk + (size_t)lvl * (size_t)E.pk_stride * 4);
 }
 // Sinks s in [0, nf + ns): s < nf -> F[s] (fast), else L[s - nf] (slow). Slow sources are
-// drifted by h on the fly; fast sinks see slow sources only. A unit is a block of T sinks
+// drifted by h on the fly; fast sinks see slow sources only. A unit is a block of 8 sinks
 // of one kind; its sums go to k_part (slow sources in slots 0-2, fast sources in 3-5).
 __device__ void kick_fp64_block(const EParams& E, const int32_t* F, const int32_t* L, int nf,
-                                int ns, double h, const double4* PK, int s0, int s1, int cs,
-                                Smem& sm) {
+                                int ns, double h, const double4* PK, int s0, int s1, Smem& sm) {
     const SoA& P = E.P;
     auto& K = sm.u.k64;
     const bool slow = s0 >= nf;
-    const int tid = threadIdx.x, T = kK64Pairs >> cs, nsink = s1 - s0;
+    const int tid = threadIdx.x, nsink = s1 - s0;
     // a slow particle at its kick position: its packed record, or drifted here
     auto drifted = [&](int q, double& x, double& y, double& z, double& m) {
         if (PK) {
@@ -1195,12 +1196,12 @@ __device__ void kick_fp64_block(const EParams& E, const int32_t* F, const int32_
         K.sx[tid] = x; K.sy[tid] = y; K.sz[tid] = z;
     }
     __syncthreads();
-    const int c = tid / T, s = tid & (T - 1);
-    const bool out = c < 3 && s < nsink;
+    const int c = kick64_component(), s = kick64_sink();
+    const bool out = c >= 0 && s < nsink;
     // one loop for both kinds of sources: a single copy of the inlined pair code
     for (int p = 0; p < (slow && nf > 0 ? 2 : 1); p++) {
         const int32_t* S = p ? F : (PK ? nullptr : L);
-        const double a = kick64_sums(K, cs, nsink, p ? nf : ns, E.eps2,
+        const double a = kick64_sums(K, nsink, p ? nf : ns, E.eps2,
                                      [&](int j) { return list_at(S, j); },
                                      [&](int g, double& x, double& y, double& z, double& m) {
                                          if (p) {
@@ -1214,32 +1215,22 @@ __device__ void kick_fp64_block(const EParams& E, const int32_t* F, const int32_
 }
 
 // Sinks [lo, hi) of the node over the workers: the slow blocks first (they see every
-// source), then the fast ones. Blocks of 8 sinks while those give the workers at most
-// kK64Rounds blocks each (the finest split; a stage's additions are then 256 long), else of
-// 32 (64 long): at N=16384 the kicks take 30.9 ms with one round, 23.8 with two or eight. PK: the slow particles packed at their kick positions (null: gathered from the
-// state arrays and drifted here). ctr: a work counter (null: blocks are dealt round robin).
-constexpr int kK64Rounds = 4;
+// source), then the fast ones. PK: the slow particles packed at their kick positions (null:
+// gathered from the state arrays and drifted here). ctr: a work counter (null: blocks are dealt
+// round robin).
 __device__ void kick_fp64_units(const EParams& E, const int32_t* F, const int32_t* L, int nf,
                                 int ns, double h, const double4* PK, int lo, int hi,
                                 unsigned* ctr, const Workers& W, Smem& sm) {
     const int f0 = min(lo, nf), f1 = min(hi, nf), l0 = max(lo, nf), l1 = max(hi, nf);
-    auto shift = [&](int cnt) { return cnt <= 8 * kK64Rounds * W.count ? 8 : 6; };
-    const int csf = shift(f1 - f0), css = shift(l1 - l0);
-    const int Tf = kK64Pairs >> csf, Ts = kK64Pairs >> css;
-    const int us = (l1 - l0 + Ts - 1) / Ts, units = us + (f1 - f0 + Tf - 1) / Tf;
-    int u = W.id;
-    if (ctr) {
-        if (threadIdx.x == 0) sm.bcast = (int)atomicAdd(ctr, 1u);
-        __syncthreads();
-        u = sm.bcast;
-    }
-    while (u < units) {
+    constexpr int T = kK64Sinks;
+    const int us = (l1 - l0 + T - 1) / T, units = us + (f1 - f0 + T - 1) / T;
+    int u = W.id;  // each worker's first unit: taken from the counter, the early workers would
+    while (u < units) {  // have the slow blocks of the late ones as their second
         __syncthreads();  // every thread has read sm.bcast
-        if (ctr && threadIdx.x == 0) sm.bcast = (int)atomicAdd(ctr, 1u);
+        if (ctr && threadIdx.x == 0) sm.bcast = W.count + (int)atomicAdd(ctr, 1u);
         const bool slow = u < us;
-        const int s0 = slow ? l0 + u * Ts : f0 + (u - us) * Tf;
-        kick_fp64_block(E, F, L, nf, ns, h, PK, s0, min(slow ? l1 : f1, s0 + (slow ? Ts : Tf)),
-                        slow ? css : csf, sm);
+        const int s0 = slow ? l0 + u * T : f0 + (u - us) * T;
+        kick_fp64_block(E, F, L, nf, ns, h, PK, s0, min(slow ? l1 : f1, s0 + T), sm);
         u = ctr ? sm.bcast : u + W.count;
     }
     __syncthreads();
@@ -3576,7 +3567,8 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 if (threadIdx.x == 0) atomicOr(E.err, HHS_ERRBIT_DEPTH);
                 return false;
             }
-            if (n <= E.mid_n && n <= kMid) {
+            if (n <= (PREC == HHS_PREC_FP64 && MODE == kModeGrid ? min(E.mid_n, kMidFp64) : E.mid_n) &&
+                n <= kMid) {
                 // the whole subtree from shared memory: on the grid's first cluster (or
                 // CTA 0), on this hardware cluster, or on this CTA alone
                 if constexpr (MODE == kModeGrid) {

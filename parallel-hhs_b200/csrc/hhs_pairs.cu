@@ -380,29 +380,25 @@ __global__ void __launch_bounds__(kKickBlock)
 
 // ---------------------------------------------------------------- standalone kicks
 // kick_slow / kick_sf of the reference API: sinks sink[0..n), sources src[0..m).
-// sinks in blocks of 8 up to here (2048 blocks), of 32 beyond: 2.84e11 against 2.66e11 pairs/s
-// at 16384 and 16400 sinks, 3.3e11 at 32768
-constexpr int kK64FineSinks = 16384;
-// FP64: a CTA per block of T = kK64Pairs >> cs sinks, terms evaluated by all its threads and
-// added in source order (hhs_kick64.cuh).
-constexpr int kK64Pairs = 2048;
+// FP64: a CTA per block of 8 sinks, terms evaluated by seven of its warps and added in source
+// order by the eighth (hhs_kick64.cuh).
 __global__ void __launch_bounds__(kK64Threads, 2)
     k_kick_pair_fp64(SoA K, double* __restrict__ ax_out, double* __restrict__ ay_out,
-                     double* __restrict__ az_out, SoA S, int n, int m, double dtfac, int cs) {
+                     double* __restrict__ az_out, SoA S, int n, int m, double dtfac) {
     extern __shared__ __align__(16) unsigned char k64_smem[];
-    auto& k = *reinterpret_cast<Kick64Smem<kK64Pairs>*>(k64_smem);
-    const int T = kK64Pairs >> cs, s0 = blockIdx.x * T, nsink = min(T, n - s0);
+    auto& k = *reinterpret_cast<Kick64Smem*>(k64_smem);
+    const int s0 = blockIdx.x * kK64Sinks, nsink = min(kK64Sinks, n - s0);
     const int tid = threadIdx.x;
     if (tid < nsink) {
         k.sx[tid] = K.x[s0 + tid]; k.sy[tid] = K.y[s0 + tid]; k.sz[tid] = K.z[s0 + tid];
     }
     __syncthreads();
-    const double a = kick64_sums(k, cs, nsink, m, 0.0, [](int j) { return j; },
+    const double a = kick64_sums(k, nsink, m, 0.0, [](int j) { return j; },
                                  [&](int j, double& x, double& y, double& z, double& mj) {
                                      x = S.x[j]; y = S.y[j]; z = S.z[j]; mj = S.m[j];
                                  });
-    const int c = tid / T, i = s0 + (tid & (T - 1));
-    if (c >= 3 || i >= n) return;
+    const int c = kick64_component(), i = s0 + kick64_sink();
+    if (c < 0 || i >= n) return;
     double* out = c == 0 ? ax_out : (c == 1 ? ay_out : az_out);
     double* v = c == 0 ? K.vx : (c == 1 ? K.vy : K.vz);
     if (out) out[i] = a;
@@ -606,12 +602,11 @@ hhs_status launch_kick_pair(const SoA& sink, double* ax, double* ay, double* az,
                             hhs_precision prec, cudaStream_t stream) {
     if (n_sink <= 0) return HHS_OK;
     if (prec == HHS_PREC_FP64) {
-        const int cs = n_sink <= kK64FineSinks ? 8 : 6;
-        constexpr int bytes = (int)sizeof(Kick64Smem<kK64Pairs>);
+        constexpr int bytes = (int)sizeof(Kick64Smem);
         HHS_CUDA_TRY(cudaFuncSetAttribute(k_kick_pair_fp64,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        k_kick_pair_fp64<<<grid_for(n_sink, kK64Pairs >> cs), kK64Threads, bytes, stream>>>(
-            sink, ax, ay, az, src, n_sink, n_src, dtfac, cs);
+        k_kick_pair_fp64<<<grid_for(n_sink, kK64Sinks), kK64Threads, bytes, stream>>>(
+            sink, ax, ay, az, src, n_sink, n_src, dtfac);
     } else
         k_kick_pair_mixed<<<grid_for(n_sink, 32), 32 * kPmWarps, 0, stream>>>(
             sink, ax, ay, az, src, n_sink, n_src, dtfac);

@@ -1,13 +1,13 @@
 """FP64 kick of a block of sinks (hhs_kick64.cuh) at the edges of its tiles: the pair terms are
 evaluated by a whole CTA and added in source order, so every sum equals the oracle's bit for
-bit (blocks of 8 sinks x stages of 256 sources up to 16384 sinks, 32 x 64 beyond)."""
+bit (blocks of 8 sinks x stages of 224 sources)."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n_sink,n_src", [(1, 1), (7, 255), (8, 256), (9, 257), (8, 513),
+@pytest.mark.parametrize("n_sink,n_src", [(1, 1), (7, 223), (8, 224), (9, 225), (8, 449),
                                           (33, 1000), (16384, 17), (16385, 63), (16417, 129)])
 def test_kick_sf_fp64_tile_edges_bit_exact(cuda, hhs, oracle, n_sink, n_src):
     sink, src = hhs.plummer(max(2, n_sink), 5), hhs.plummer(max(2, n_src), 6)
