@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <array>
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <new>
@@ -42,6 +43,7 @@
 #include "hhs_pairmath.cuh"
 #include "hhs_scan.cuh"
 #include "hhs_tma.cuh"
+#include "hhs_tsrows.cuh"
 
 using namespace hhs;
 
@@ -195,6 +197,7 @@ struct __align__(16) Smem {
         struct { float4 A[kEB], B[kEB], V[kEB]; } tsm;         // mixed timestep tiles
         struct { double x[kEB], y[kEB], z[kEB], vx[kEB], vy[kEB], vz[kEB], m[kEB]; } tsd;
         struct { float4 A[kEB], B[kEB]; } km;                   // mixed kick tiles
+        TsRows tr;                                              // timesteps by rows
         struct { float4 A[kTS], B[kTS]; } kt;                   // grid kick source tile
         struct {                                                  // symmetric kick
             float4 T[2][kTX / 2][4];                              // source pairs
@@ -2134,37 +2137,22 @@ __device__ void kick_unit_x2(const EParams& E, const int32_t* F, const int32_t* 
 }
 
 // ---------------------------------------------------------------- node phases
-// Per-sink reduction of the timestep partials (calc) or plain predicate (no calc),
-// writing per-tile predicate counts.
+// Timesteps from the rate words (mixed, calc) and predicate counts per tile.
 template <int PREC>
 __device__ void count_phase(const EParams& E, const int32_t* S, int n, double dt, bool calc,
-                            int nch, const Workers& W, Smem& sm) {
+                            const Workers& W, Smem& sm) {
     const int ntiles = (n + kEB - 1) / kEB;
     for (int t = W.id; t < ntiles; t += W.count) {
         const int i = t * kEB + threadIdx.x;
         int flag = 0;
         if (i < n) {
             const int gi = list_at(S, i);
-            double ts;
-            if (calc) {
-                if (PREC == HHS_PREC_FP64) {
-                    double mv = 1.e30;
-                    for (int c = 0; c < nch; c++) {
-                        const double v = E.ts_part[(size_t)c * E.n_max + i];
-                        if (v < mv) mv = v;
-                    }
-                    ts = mv;
-                } else {
-                    const float mr = __uint_as_float(E.rate_acc[i]);
-                    E.rate_acc[i] = 0u;
-                    const double tv = 1.0 / (double)mr;
-                    ts = tv < 1.e30 ? tv : 1.e30;
-                }
-                E.P.ts[gi] = ts;
-            } else {
-                ts = E.P.ts[gi];
+            if (PREC != HHS_PREC_FP64 && calc) {
+                const double tv = 1.0 / (double)__uint_as_float(E.rate_acc[i]);
+                E.rate_acc[i] = 0u;
+                E.P.ts[gi] = tv < 1.e30 ? tv : 1.e30;
             }
-            flag = ts <= dt;
+            flag = E.P.ts[gi] <= dt;
         }
         const int c = block_sum(flag, sm);
         if (threadIdx.x == 0) E.tile_counts[t] = c;
@@ -3209,8 +3197,8 @@ __device__ void warp_subtree(const EParams& E, MidState& M, const unsigned* memw
 // cs, rank: the hardware cluster that runs the subtree (every CTA of it calls mid_hold),
 // or cs = 1 for one CTA alone whatever cluster it belongs to.
 template <int PREC>
-__device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int n, int level0, bool calc0,
-                         int dist_n, int cs, int rank) {
+__device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int n, int level0,
+                                         bool calc0, int dist_n, int cs, int rank) {
     Smem& sm = cta_smem();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -3534,6 +3522,13 @@ __device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int
     mid_mark(E, sm, tm, 61);
 }
 
+// The FP64 solver as a function: the batched kernel has it in three places, and inlined in each
+// it spills (300 systems of up to 640 particles: 9.9 ms, called 9.1).
+__device__ __noinline__ void mid_hold_fp64(const EParams& E, const int32_t* S, int n, int level0,
+                                           bool calc0, int dist_n, int cs, int rank) {
+    mid_hold<HHS_PREC_FP64>(E, S, n, level0, calc0, dist_n, cs, rank);
+}
+
 // True when the kick of level lvl (a grid node with a fast set of at most mid_n) runs its
 // slow-only units beside the fast set's first pass on the first cluster: mixed precision,
 // packed sources at that level, and CTAs outside the first cluster.
@@ -3587,7 +3582,10 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                                        1, sm);
                     }
                 } else {
-                    mid_hold<PREC>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
+                    if constexpr (PREC == HHS_PREC_FP64)
+                        mid_hold_fp64(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
+                    else
+                        mid_hold<PREC>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfCluster, 0.0, sm, lvl);
@@ -3650,7 +3648,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                             ts_filter_merge<PREC>(E, S, n, rbn, cw, u, sm);
                         }
                     }
-                } else if (PREC == HHS_PREC_FP64) {
+                } else if (MODE == kModeGrid) {  // FP64
                     nch = chunks_for(n, W, true, E.units_per_cta);
                     const int C = (n + nch - 1) / nch;
                     const int nsb = (n + kEB - 1) / kEB;
@@ -3660,10 +3658,25 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                         ts_unit<PREC>(E, S, n, ib, j0, j1, E.ts_part + (size_t)jc * E.n_max,
                                       nullptr, sm);
                     }
+                } else if (PREC == HHS_PREC_FP64) {
+                    // blocks of rows over the workers (one CTA, or the cluster's), as many rows
+                    // as leave no worker idle
+                    const TsArgs A{E.eta, E.eta_s2, E.inv_eta_s2, E.inv_eta};
+                    int T = kTsMaxRows;
+                    while (T > 8 && (n + T - 1) / T < W.count) T >>= 1;
+                    for (int i0 = W.id * T; i0 < n; i0 += W.count * T) {
+                        const int nrow = min(T, n - i0);
+                        ts_rows<PREC>(E.P, S, n, i0, nrow, A, sm.u.tr);
+                        if ((int)threadIdx.x < nrow)
+                            E.P.ts[list_at(S, i0 + threadIdx.x)] =
+                                ts_of_key<PREC>(sm.u.tr.best[threadIdx.x]);
+                        __syncthreads();
+                    }
                 } else {
                     // only units with a pair j > i: row block rb takes column blocks
                     // cb >= rb * kEB / kCB; each worker takes a contiguous range of that
-                    // triangle in row-major order
+                    // triangle in row-major order (the rows with their filter, as in FP64, take
+                    // 40 ms against 33 for 512 clusters: a CTA alone waits for every tile)
                     const long long units = ts_sym_units(n);
                     const int u0 = (int)(units * W.id / W.count);
                     const int u1 = (int)(units * (W.id + 1) / W.count);
@@ -3675,7 +3688,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
             if constexpr (MODE == kModeGrid) {
                 split_phase<PREC, FILTER>(E, S, n, dt, lvl, calc, nch, filtered, lvl == top, W, sm);
             } else {
-                count_phase<PREC>(E, S, n, dt, calc, nch, W, sm);
+                count_phase<PREC>(E, S, n, dt, calc, W, sm);
                 if (!phase_barrier(E, sm, W)) return false;
                 scatter_phase(E, S, n, dt, lvl, calc, W, sm);
             }
@@ -4588,7 +4601,7 @@ struct hhs_batch {
     hhs_params params{0.03, 0.0};
     int big_n = 1024, cluster_size = 8, small_n = 64, units_per_cta = 8, warp_n = 32, packed = 0;
     int mid_n = kMid, mid_dist_n = 96;
-    int n_big = 0, n_clusters[2] = {0, 0};
+    int n_big = 0, n_big64 = 0, n_clusters[2] = {0, 0};  // n_big64: FP64 steps
     void* arena = nullptr;
     int32_t* d_offsets = nullptr;
     int32_t* d_order = nullptr;
@@ -4610,6 +4623,10 @@ cudaError_t batched_occupancy(int cs, int* clusters) {
     cudaError_t e = cudaFuncSetAttribute(k_batched<PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kEngineSmem);
     if (e != cudaSuccess) return e;
+    if (cs > 8) {
+        e = cudaFuncSetAttribute(k_batched<PREC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs, 1, 1);
     cfg.blockDim = dim3(kEB, 1, 1);
@@ -4622,6 +4639,32 @@ cudaError_t batched_occupancy(int cs, int* clusters) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaOccupancyMaxActiveClusters(clusters, (void*)k_batched<PREC>, &cfg);
+}
+
+// Clusters of the launch, and the size above which a system gets a cluster, from the systems'
+// sizes. e is the number of systems of the largest one's cost (n^2.33, the pairs of a step) that
+// the large systems add up to. Few of them: the launch is as long as the largest system, so each
+// gets 16 CTAs; many: the launch is bound by throughput, which small clusters have most of (their
+// barriers span fewer CTAs and more systems run side by side). Measured, ms per launch with
+// clusters of 4 / 8 / 16: 32 systems of 64 to 4096 particles (e = 3.3) 16.2 / 11.1 / 6.8, 100
+// (10) 21.6 / 11.6 / 11.8, 200 (21) 23.6 / 13.5 / 18.9, 512 (53) 26.0 / 32.3 / 47.2; 300 of 64 to
+// 2048 (37) 10.4 / 9.8 / 12.8. Where no system exceeds 1024 particles, those above 640 (the largest
+// that one CTA holds in shared memory) get the clusters: 500 systems of 64 to 1024 (51) 3.6 ms
+// with clusters of 4 against 4.6 with every system on a CTA of its own.
+bool batched_shape(hhs_batch* b, int* c0, int* c1) {
+    b->big_n = b->n_max_sys > 1024 ? 1024 : kMid;
+    double e = 0.0;
+    for (const int n : b->sizes)
+        if (n > b->big_n) e += std::pow((double)n / b->n_max_sys, 2.33);
+    // the portable size is the fallback
+    for (const int cs : {e < 8.0 ? 16 : (e < 40.0 ? 8 : 4), 8}) {
+        b->cluster_size = cs;
+        if (batched_occupancy<HHS_PREC_FP64>(cs, c0) == cudaSuccess &&
+            batched_occupancy<HHS_PREC_MIXED>(cs, c1) == cudaSuccess && *c0 > 0 && *c1 > 0)
+            return true;
+        (void)cudaGetLastError();
+    }
+    return false;
 }
 
 size_t slot_layout(int n, int levels, int chunks, size_t* off) {
@@ -4659,13 +4702,8 @@ extern "C" hhs_status hhs_batch_create(int32_t n_sys, const int32_t* offsets, in
     std::iota(b->order.begin(), b->order.end(), 0);
     std::stable_sort(b->order.begin(), b->order.end(),
                      [&](int a, int c) { return b->sizes[a] > b->sizes[c]; });
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int c0 = 0, c1 = 0;
-    if (batched_occupancy<HHS_PREC_FP64>(b->cluster_size, &c0) != cudaSuccess ||
-        batched_occupancy<HHS_PREC_MIXED>(b->cluster_size, &c1) != cudaSuccess || c0 <= 0 ||
-        c1 <= 0) {
+    if (!batched_shape(b, &c0, &c1)) {
         delete b;
         return HHS_ERR_CUDA;
     }
@@ -4704,8 +4742,12 @@ extern "C" hhs_status hhs_batch_create(int32_t n_sys, const int32_t* offsets, in
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_order, b->order.data(), sizeof(int32_t) * n_sys, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { cudaFree(b->arena); delete b; return hhs_from_cuda(e); }
-    for (int k = 0; k < n_sys; k++)
+    // FP64 systems that one CTA does not hold in shared memory get a cluster unless the caller's
+    // tuning says otherwise (400 systems of 64 to 2048: 34.5 ms, with 1024 as in mixed 41.5)
+    for (int k = 0; k < n_sys; k++) {
         if (b->sizes[b->order[k]] > b->big_n) b->n_big = k + 1;
+        if (b->sizes[b->order[k]] > kMid) b->n_big64 = k + 1;
+    }
     *out = b;
     return HHS_OK;
 }
@@ -4727,6 +4769,7 @@ extern "C" hhs_status hhs_batch_set_tuning(hhs_batch* b, int32_t big_n, int32_t 
     b->n_big = 0;
     for (int k = 0; k < b->n_sys; k++)
         if (b->sizes[b->order[k]] > b->big_n) b->n_big = k + 1;
+    b->n_big64 = b->n_big;
     return HHS_OK;
 }
 
@@ -4795,7 +4838,7 @@ extern "C" hhs_status hhs_hold_batched(hhs_batch* b, hhs_particle_system* sys, d
     B.offsets = b->d_offsets;
     B.order = b->d_order;
     B.n_sys = b->n_sys;
-    B.n_big = b->n_big;
+    B.n_big = pi == 0 ? b->n_big64 : b->n_big;
     B.queues = b->d_queues;
     B.cluster_slots = b->cluster_slots;
     B.cta_slots = b->cta_slots;

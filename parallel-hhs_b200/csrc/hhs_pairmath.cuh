@@ -55,7 +55,7 @@ __device__ __forceinline__ void kick_pair_fp64(double dx, double dy, double dz, 
         f64_add(f64_add(f64_mul(dx, dx), f64_mul(dy, dy)), f64_mul(dz, dz)), eps2);
     if (d2 == 0.0) return;
     const double d = f64_sqrt(d2);
-    const double s = f64_mul(mj, f64_div(1.0, f64_mul(d2, d)));
+    const double s = f64_mul(mj, __drcp_rn(f64_mul(d2, d)));  // 1 / (d2 d), the same rounding
     ax = f64_add(ax, f64_mul(dx, s));
     ay = f64_add(ay, f64_mul(dy, s));
     az = f64_add(az, f64_mul(dz, s));

@@ -1,0 +1,221 @@
+// hhs_tsrows.cuh -- timesteps of a block of particles by one CTA, in either precision: the
+// standalone timesteps call and the batched step's nodes (the device step's grid nodes have
+// their own form, over pairs, in hhs_engine.cu).
+#pragma once
+#include "hhs_common.cuh"
+#include "hhs_pairmath.cuh"
+
+namespace hhs {
+
+constexpr double kHuge = 1.e30;  // src/timestep.cuh:4
+
+__device__ __forceinline__ int ts_list_at(const int32_t* list, int i) { return list ? list[i] : i; }
+
+// A CTA takes T rows (particles) and passes over all n columns, 512 at a time, two a thread in
+// registers, with the pair test of the device step's filtered timestep (hhs_engine.cu): a pair
+// below a row's best rate so far is left out by 9 packed FP32 operations for two pairs, and the
+// few that pass are listed and evaluated exactly, in either precision, some dozens at a time.
+// Each row starts from its exact rates over the first 32 columns. The result is the maximum
+// over all pairs, as if every one had been evaluated.
+//
+// The test here is for the row alone, with its rate T = 0.99 best: a pair may be left out if
+//     A >= kappa B + C (p_i + p_j) and B >= D (p_i + p_j),  p = |m|^(2/3),
+// A = |x_i - x_j|^2, B = |v_i - v_j|^2, C = (2 / (eta beta T)^2)^(2/3), D = (1 / (2 (1 - alpha)
+// T C))^2: C (p_i + p_j) is at least the `a` and D (p_i + p_j) at least the `b` of the pair's
+// mass sum there, since (m_i + m_j)^(2/3) <= p_i + p_j.
+//
+// Measured, one call: 2051 particles in FP64 1384 -> 23 us, 16384 mixed 1652 -> 261 us. What
+// bounds it: the latency of a row's test (a chain of six packed operations, its shared-memory
+// reads and a branch, hidden by eight warps per scheduler at most), and below about 4000
+// particles that of a tile's loads and listed pairs.
+constexpr int kTsThreads = 256;
+constexpr int kTsCols = 2 * kTsThreads;  // columns of a tile
+constexpr int kTsSeed = 32;              // columns that every row evaluates first
+constexpr int kTsCap = 2048;             // pairs listed at a time
+constexpr unsigned kTsBatch = 64;        // listed pairs that are worth evaluating together
+constexpr int kTsMaxRows = 32;
+constexpr float kTsAlpha = 0.9f;
+constexpr float kTsAll = 1.0e38f;
+
+struct __align__(16) TsRowTest {  // -2 x, -2 v, -kappa, -C, -D, each in both lanes; pass: v <= c1 or w < c2
+    float2 x, y, z, vx, vy, vz, nk, nC, nD;
+    float c1, c2;
+};
+
+struct TsArgs {
+    double eta, eta_s2;
+    float inv_eta_s2, inv_eta;
+};
+
+struct TsState {
+    double x, y, z, vx, vy, vz, m;
+};
+
+__device__ __forceinline__ TsState ts_load(const SoA& P, int g) {
+    return TsState{P.x[g], P.y[g], P.z[g], P.vx[g], P.vy[g], P.vz[g], P.m[g]};
+}
+
+// the pair's rate as FP32 bits (mixed) or the complement of its timescale's bits (FP64): the
+// largest key is the timestep; 0 for none
+template <int PREC>
+__device__ __forceinline__ unsigned long long ts_key(const TsState& a, const TsState& b,
+                                                     const TsArgs& A) {
+    if constexpr (PREC == HHS_PREC_FP64) {
+        double t = kHuge;
+        ts_pair_fp64(f64_sub(a.x, b.x), f64_sub(a.y, b.y), f64_sub(a.z, b.z), f64_sub(a.vx, b.vx),
+                     f64_sub(a.vy, b.vy), f64_sub(a.vz, b.vz), a.m, b.m, A.eta, A.eta_s2, t);
+        return t < kHuge ? ~(unsigned long long)__double_as_longlong(t) : 0ull;
+    } else {
+        const DS ax = ds_split(a.x), ay = ds_split(a.y), az = ds_split(a.z);
+        const DS bx = ds_split(b.x), by = ds_split(b.y), bz = ds_split(b.z);
+        const float r = ts_pair_rate_mixed(
+            ds_diff(ax.hi, ax.lo, bx.hi, bx.lo), ds_diff(ay.hi, ay.lo, by.hi, by.lo),
+            ds_diff(az.hi, az.lo, bz.hi, bz.lo), (float)a.vx - (float)b.vx,
+            (float)a.vy - (float)b.vy, (float)a.vz - (float)b.vz, (float)a.m + (float)b.m,
+            A.inv_eta_s2, A.inv_eta);
+        return r > 0.0f ? (unsigned long long)__float_as_uint(r) : 0ull;
+    }
+}
+template <int PREC>
+__device__ __forceinline__ double ts_of_key(unsigned long long key) {
+    if (key == 0ull) return kHuge;
+    if (PREC == HHS_PREC_FP64) return __longlong_as_double((long long)~key);
+    const double t = 1.0 / (double)__uint_as_float((unsigned)key);
+    return t < kHuge ? t : kHuge;
+}
+
+template <int PREC>
+__device__ __forceinline__ TsRowTest ts_row_test(const TsState& q, unsigned long long key,
+                                                 const TsArgs& A) {
+    TsRowTest r;
+    const double rate = 1.0 / ts_of_key<PREC>(key), r2 = q.x * q.x + q.y * q.y + q.z * q.z,
+                 v2 = q.vx * q.vx + q.vy * q.vy + q.vz * q.vz;
+    const float T = 0.99f * (float)rate, eta = (float)A.eta;
+    const float e = 1.0f / eta + 0.5f, beta = 1.0f - 0.75f * kTsAlpha / e;
+    const float k = e / (kTsAlpha * T), f = eta * beta * T, c = cbrtf(2.01f / (f * f));
+    const float kappa = 1.01f * k * k, C = 1.02f * c * c;
+    const float h = 0.5f / ((1.0f - kTsAlpha) * T * C), D = 1.02f * h * h;
+    const float pm = cbrtf((float)fabs(q.m)), p = 1.01f * pm * pm;
+    const float W = (float)(r2 * (1.0 - 4e-6)), U = (float)(v2 * (1.0 + 4e-6));
+    // without a usable rate (or for eta beyond the test's range) every pair passes
+    const bool ok = A.eta <= 1.0 && rate > 1e-12 && rate < 1e12 && r2 < 1e24 && v2 < 1e24 &&
+                    kappa < 1e24f && C * p < 1e24f && D * p < 1e24f;
+    r.x = f2dup(ok ? -2.0f * (float)q.x : 0.0f);
+    r.y = f2dup(ok ? -2.0f * (float)q.y : 0.0f);
+    r.z = f2dup(ok ? -2.0f * (float)q.z : 0.0f);
+    r.vx = f2dup(ok ? -2.0f * (float)q.vx : 0.0f);
+    r.vy = f2dup(ok ? -2.0f * (float)q.vy : 0.0f);
+    r.vz = f2dup(ok ? -2.0f * (float)q.vz : 0.0f);
+    r.nk = f2dup(ok ? -kappa : 0.0f);
+    r.nC = f2dup(ok ? -C : 0.0f);
+    r.nD = f2dup(ok ? -D : 0.0f);
+    const float a = C * p + 1e-30f;
+    r.c1 = ok ? (a - W + kappa * U) + 2e-6f * (a + W + kappa * U) : 3e38f;
+    r.c2 = ok ? D * p + 4e-5f * U + 1e-30f - U : 3e38f;
+    return r;
+}
+
+struct TsRows {  // shared memory of ts_rows
+    TsState row[kTsMaxRows];
+    TsRowTest test[kTsMaxRows];
+    unsigned long long best[kTsMaxRows];
+    int2 hit[kTsCap];  // (row, column)
+    unsigned cnt;
+};
+
+// The keys of rows i0 .. i0 + nrow - 1 (at most kTsMaxRows) of the n particles of `list` into
+// sm.best. Called by all kTsThreads threads of the CTA; ends with a CTA barrier.
+template <int PREC>
+__device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n, int i0, int nrow,
+                                        const TsArgs& A, TsRows& sm) {
+    const int tid = threadIdx.x;
+    if (tid < nrow) sm.row[tid] = ts_load(P, ts_list_at(list, i0 + tid));
+    if (tid < kTsMaxRows) sm.best[tid] = 0ull;
+    if (tid == 0) sm.cnt = 0u;
+    __syncthreads();
+    for (int k = tid; k < nrow * kTsSeed; k += kTsThreads) {
+        const int r = k / kTsSeed, j = k % kTsSeed;
+        if (j < n && j != i0 + r) {
+            const unsigned long long q = ts_key<PREC>(sm.row[r], ts_load(P, ts_list_at(list, j)), A);
+            if (q > sm.best[r]) atomicMax(&sm.best[r], q);
+        }
+    }
+    __syncthreads();
+    if (tid < nrow) sm.test[tid] = ts_row_test<PREC>(sm.row[tid], sm.best[tid], A);
+    __syncthreads();
+    unsigned held = 0u;
+    for (int t0 = 0; t0 < n; t0 += kTsCols) {
+        const int j0 = t0 + 2 * tid;
+        float2 X, Y, Z, VX, VY, VZ, W, U, p;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const TsState q = j0 + c < n ? ts_load(P, ts_list_at(list, j0 + c))
+                                         : TsState{0, 0, 0, 0, 0, 0, 0};
+            const double r2 = q.x * q.x + q.y * q.y + q.z * q.z,
+                         v2 = q.vx * q.vx + q.vy * q.vy + q.vz * q.vz;
+            const float pm = cbrtf((float)fabs(q.m)), pc = 1.01f * pm * pm;
+            const bool ok = r2 < 1e24 && v2 < 1e24 && pc < 1e20f;  // else it passes every test
+            auto put = [&](float2& v, float f) {
+                if (c) v.y = f;
+                else v.x = f;
+            };
+            put(X, ok ? (float)q.x : 0.0f);
+            put(Y, ok ? (float)q.y : 0.0f);
+            put(Z, ok ? (float)q.z : 0.0f);
+            put(VX, ok ? (float)q.vx : 0.0f);
+            put(VY, ok ? (float)q.vy : 0.0f);
+            put(VZ, ok ? (float)q.vz : 0.0f);
+            put(p, ok ? pc : 0.0f);
+            put(W, ok ? (float)(r2 * (1.0 - 4e-6)) : -kTsAll);
+            put(U, ok ? (float)(v2 * (1.0 + 4e-6)) : 0.0f);
+        }
+        for (int r = 0; r < nrow; r++) {
+            __syncwarp();  // lanes that listed pairs rejoin the others here
+            const TsRowTest t = sm.test[r];
+            float2 w = __ffma2_rn(t.vx, VX, U), v = __ffma2_rn(t.x, X, W);
+            w = __ffma2_rn(t.vy, VY, w);
+            v = __ffma2_rn(t.y, Y, v);
+            w = __ffma2_rn(t.vz, VZ, w);
+            v = __ffma2_rn(t.z, Z, v);
+            v = __ffma2_rn(t.nk, w, v);
+            v = __ffma2_rn(t.nC, p, v);
+            w = __ffma2_rn(t.nD, p, w);
+            if (fminf(v.x, v.y) <= t.c1 || fminf(w.x, w.y) < t.c2) {
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const float vc = c ? v.y : v.x, wc = c ? w.y : w.x;
+                    if ((vc <= t.c1 || wc < t.c2) && j0 + c < n && j0 + c != i0 + r) {
+                        const unsigned k = atomicAdd(&sm.cnt, 1u);
+                        if (k < kTsCap) sm.hit[k] = make_int2(r, j0 + c);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        const unsigned cnt = sm.cnt;
+        __syncthreads();  // every thread has the count
+        if (cnt < kTsBatch && t0 + kTsCols < n) {
+            held = cnt;
+            continue;
+        }
+        // the listed pairs; if the list overflowed, those of earlier tiles and every pair of
+        // this one
+        const bool all = cnt > kTsCap;
+        const int listed = (int)(all ? held : cnt), total = listed + (all ? nrow * kTsCols : 0);
+        for (int k = tid; k < total; k += kTsThreads) {
+            const int2 h = k < listed ? sm.hit[k]
+                                      : make_int2((k - listed) / kTsCols, t0 + (k - listed) % kTsCols);
+            if (h.y >= n || h.y == i0 + h.x) continue;
+            const unsigned long long key =
+                ts_key<PREC>(sm.row[h.x], ts_load(P, ts_list_at(list, h.y)), A);
+            if (key > *(volatile unsigned long long*)&sm.best[h.x]) atomicMax(&sm.best[h.x], key);
+        }
+        __syncthreads();
+        if (tid == 0) sm.cnt = 0u;
+        if (tid < nrow) sm.test[tid] = ts_row_test<PREC>(sm.row[tid], sm.best[tid], A);
+        __syncthreads();
+        held = 0u;
+    }
+}
+
+}  // namespace hhs
