@@ -3795,6 +3795,24 @@ __global__ void __launch_bounds__(kEB, 2) k_engine(const __grid_constant__ EPara
     prof_end(E, sm);
 }
 
+// A system that the subtree solver takes whole: one cluster instead of a cooperative launch of the
+// whole GPU with its barrier and look-back words cleared first, and a kernel without the grid
+// phases' registers (256 particles: 319 -> 290 us). What bounds it is the solver's latency: over a
+// hundred nodes one after another, most of them on one warp.
+template <int PREC>
+__global__ void __launch_bounds__(kEB, 1) k_subtree(const __grid_constant__ EParams E) {
+    Smem& sm = cta_smem();
+    namespace cg = cooperative_groups;
+    const Workers W{(int)blockIdx.x, (int)gridDim.x, kModeGrid};
+    unsigned long long t_last = 0;
+    prof_begin(E, sm);
+    prof_mark(E, W, t_last, -1, 0.0, sm);
+    mid_hold<PREC>(E, nullptr, E.n_top, 0, E.calc_top != 0, E.mid_dist_n,
+                   (int)cg::this_cluster().num_blocks(), (int)cg::this_cluster().block_rank());
+    prof_mark(E, W, t_last, kProfCluster, 0.0, sm, 0);
+    prof_end(E, sm);
+}
+
 // Probe of the mixed grid kick: the system as one split node whose fast set is every
 // third particle (index % 3 == 0) and whose slow set is the rest, with no drift. The
 // level's slow records are packed, the symmetric kick runs its units, and the reduce
@@ -4137,9 +4155,10 @@ inline size_t al(size_t v) { return (v + kAl - 1) & ~(kAl - 1); }
 
 namespace {
 // the kernels of the device step
-std::array<const void*, 3> engine_kernels() {
+std::array<const void*, 5> engine_kernels() {
     return {(const void*)k_engine<HHS_PREC_FP64, true>, (const void*)k_engine<HHS_PREC_MIXED, false>,
-            (const void*)k_engine<HHS_PREC_MIXED, true>};
+            (const void*)k_engine<HHS_PREC_MIXED, true>, (const void*)k_subtree<HHS_PREC_FP64>,
+            (const void*)k_subtree<HHS_PREC_MIXED>};
 }
 // Mixed steps filter their timesteps from here on: at 16384 particles the filter saves 1.9 of 4.1
 // ms of timesteps, at 4099 0.04 of 0.41, and its code costs the subtree solver in the same kernel
@@ -4452,6 +4471,24 @@ cudaError_t engine_launch(EngineHost* eh, int pi, K kernel, const EParams& E, cu
     if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kernel, E);
     return e;
 }
+
+// One cluster of the context's size on the subtree solver.
+template <class K>
+cudaError_t subtree_launch(EngineHost* eh, K kernel, const EParams& E, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(eh->cluster_size, 1, 1);
+    cfg.blockDim = dim3(kEB, 1, 1);
+    cfg.dynamicSmemBytes = kEngineSmem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = eh->cluster_size;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, E);
+}
 }  // namespace
 
 hhs_status engine_hold_step(hhs_ctx* c, const SoA& P, int n, double dt, bool calc_ts,
@@ -4463,7 +4500,11 @@ hhs_status engine_hold_step(hhs_ctx* c, const SoA& P, int n, double dt, bool cal
     EParams E = engine_params(c, eh, P, n, dt, calc_ts, profile, top_level);
     const int pi = prec == HHS_PREC_FP64 ? 0 : 1;
     E.prec_mixed = pi;
-    const cudaError_t e = pi == 0 ? engine_launch(eh, 0, k_engine<HHS_PREC_FP64, true>, E, stream)
+    const int mid_n = std::min(pi == 0 ? std::min(eh->mid_n, kMidFp64) : eh->mid_n, kMid);
+    const cudaError_t e = top_level == 0 && n <= mid_n
+                              ? (pi == 0 ? subtree_launch(eh, k_subtree<HHS_PREC_FP64>, E, stream)
+                                         : subtree_launch(eh, k_subtree<HHS_PREC_MIXED>, E, stream))
+                          : pi == 0 ? engine_launch(eh, 0, k_engine<HHS_PREC_FP64, true>, E, stream)
                           : n < kFilterN
                               ? engine_launch(eh, 1, k_engine<HHS_PREC_MIXED, false>, E, stream)
                               : engine_launch(eh, 1, k_engine<HHS_PREC_MIXED, true>, E, stream);
