@@ -1915,7 +1915,10 @@ __device__ void kick_slow_unit(const EParams& E, int nf, int lvl, const KickPlan
             E.k_part[(size_t)(jc * 3 + k) * nmx + nf + qs] = (double)acc[k] - (double)cmp[k];
 }
 
-// Units of one kind set, taken from the level's counter `set` until none is left:
+// Units of one kind set: worker `rank` of `count` starts with unit `rank` and takes the next ones
+// from the level's counter `set` until none is left (with the first unit from the counter too,
+// the workers that arrive early take two before the late ones take one: 5% of a step more at
+// 65536 and at 4099 particles, 1.5% at 16384).
 // kinds 0 = cross units then slow units, 1 = slow units only, 2 = cross units only.
 // While a unit computes, thread 0 already takes the next unit and starts the copy of its
 // first tile into the other buffer.
@@ -1935,7 +1938,8 @@ __device__ __forceinline__ void unit_first_tile(const KickPlan& p, int nx, int u
 }
 
 __device__ void kick_sym_units(const EParams& E, const int32_t* F, int nf, int ns, int lvl,
-                               const KickPlan& plan, int set, int kinds, Smem& sm) {
+                               const KickPlan& plan, int set, int kinds, int rank, int count,
+                               Smem& sm) {
     const int nx = kinds == 1 ? 0 : plan.nx;
     const int total = nx + (kinds == 2 ? 0 : plan.nsl);
     if (threadIdx.x == 0) sm.kp = plan;  // read back after each barrier below
@@ -1947,9 +1951,7 @@ __device__ void kick_sym_units(const EParams& E, const int32_t* F, int nf, int n
     tc.pending[0] = tc.pending[1] = false;
     tc.phase = sm.tphase;
     __syncthreads();  // every thread has read sm.tphase and the previous phase's sm.bcast
-    if (threadIdx.x == 0) sm.bcast = (int)atomicAdd(ctr, 1u);
-    __syncthreads();
-    int u = sm.bcast, c = 0;
+    int u = rank, c = 0;  // worker `rank` of `count`: the first unit is its own
     auto clip = [&](int& a, int& b) { b = min(b, ns); };
     if (u < total) {
         int a, b;
@@ -1961,7 +1963,7 @@ __device__ void kick_sym_units(const EParams& E, const int32_t* F, int nf, int n
     while (u < total) {
         __syncthreads();  // every thread has read sm.bcast
         if (threadIdx.x == 0) {
-            const int un = (int)atomicAdd(ctr, 1u);
+            const int un = count + (int)atomicAdd(ctr, 1u);
             sm.bcast = un;
             if (un < total) {
                 int a, b;
@@ -3579,7 +3581,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                         const int pnf = n, pns = ld_volatile_i32(&E.counts[pl].n_slow);
                         const KickPlan kp = kick_plan(pnf, pns, W.count);
                         kick_sym_units(E, E.fast_lists + (size_t)pl * E.n_max, pnf, pns, pl, kp, 1,
-                                       1, sm);
+                                       1, W.id - cs, W.count - cs, sm);
                     }
                 } else {
                     if constexpr (PREC == HHS_PREC_FP64)
@@ -3729,7 +3731,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     const bool overlapped = nf > 0 && nf <= E.mid_n && nf <= kMid &&
                                             kick_overlaps(E, lvl, W);
                     kp = kick_plan(nf, ns, W.count);
-                    kick_sym_units(E, F, nf, ns, lvl, kp, 0, overlapped ? 2 : 0, sm);
+                    kick_sym_units(E, F, nf, ns, lvl, kp, 0, overlapped ? 2 : 0, W.id, W.count, sm);
                 }
                 if constexpr (PREC == HHS_PREC_FP64) {
                     unsigned* ctr = MODE == kModeGrid ? &E.st->kick_ctr[0][lvl] : nullptr;
@@ -3849,7 +3851,7 @@ __global__ void __launch_bounds__(kEB, 2) k_engine_accel(EParams E) {
     if (W.id == 0 && threadIdx.x == 0) E.st->kick_ctr[0][0] = 0u;
     if (!grid_barrier(E, sm)) return;
     const KickPlan kp = kick_plan(nf, ns, W.count);
-    kick_sym_units(E, F, nf, ns, 0, kp, 0, 0, sm);
+    kick_sym_units(E, F, nf, ns, 0, kp, 0, 0, W.id, W.count, sm);
     if (!grid_barrier(E, sm)) return;
     double* out[3] = {E.ts_part, reinterpret_cast<double*>(E.rate_acc),
                       reinterpret_cast<double*>(E.tile_counts)};
