@@ -284,7 +284,7 @@ hhs_status hhs_ipc_close(hhs_particle_system* view);
 
 /* Exact exclusive prefix sum of int32 values (the contract of
  * scan_predicate_small/large, src/split.cuh:438-565): one decoupled-lookback pass below
- * 2^22 values, two passes over chunks (chunk sums, then chunk scans) up to 2^25, and from
+ * 2^18 values, two passes over chunks (chunk sums, then chunk scans) up to 2^25, and from
  * 2^25 values (16-byte aligned input and output) one streamed pass: a cooperative launch
  * of resident CTAs that bulk-copy chunks into shared memory and exchange chunk
  * aggregates two rounds ahead (unaligned pointers keep the two-pass form).
@@ -326,7 +326,7 @@ hhs_status hhs_scan_noalloc_selftest_stalled_predecessor(const int32_t* d_in, in
 /* Stream compaction (the split of a flag array, src/split.cuh:573-610 on int32 data):
  * d_idx[k] = index of the k-th nonzero flag, *d_count = number of nonzero flags, and
  * d_scan (optional, NULL = not written) = exclusive scan of (flag != 0). One pass below
- * 2^22 flags; from there on chunk sums then chunk scans (from 2^24 flags in one
+ * 2^18 flags; from there on chunk sums then chunk scans (from 2^24 flags in one
  * cooperative launch, in waves of 2^24 flags). Workspace as for hhs_scan_exclusive_i32. */
 hhs_status hhs_compact_flags_i32(const int32_t* d_flags, int32_t* d_scan, int32_t* d_idx,
                                  int32_t* d_count, int64_t n, void* d_workspace,

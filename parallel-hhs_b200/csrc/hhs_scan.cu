@@ -64,14 +64,21 @@ __global__ void __launch_bounds__(kScanBlock, 6)
     if (SELF_RESET && scan_finish_is_last(hdr, num_tiles, &s_last)) scan_reset(hdr, epoch);
 }
 
-// Large inputs (n >= 2^22). The single pass is held back by how fast the inclusive
+// Large inputs. The single pass is held back by how fast the inclusive
 // prefixes propagate through hundreds of resident tiles, so large inputs are scanned in
 // two steps over contiguous chunks of whole tiles, one chunk per CTA: sum the chunk,
 // then scan it from the sum of the chunks before it.
 //  - Two-kernel form: a chunk-sum kernel and a chunk-scan kernel over the whole input,
-//    12 bytes of DRAM traffic per value. The default for the scan from 2^22 values up to
+//    12 bytes of DRAM traffic per value. The default for the scan from 2^18 values up to
 //    the streamed pass below (4.25 TB/s at 2^28, where the streamed pass reaches 5.0), and
-//    for unaligned inputs.
+//    for unaligned inputs. Below 2^22 the input stays in L2 between the kernels and what
+//    counts is the chain of look-backs, which the two kernels do not have. Microseconds,
+//    single pass (with its memset) / two kernels: scan 7.8/10.4 at 2^17, 8.4/8.2 at 2^18,
+//    10.1/8.2 at 2^19, 12.3/8.2 at 2^20, 15.2/10.3 at 2^21, equal at 2^22; compaction
+//    8.3/8.4, 10.2/8.2, 11.2/8.2, 15.3/10.3 and 17.3/10.4 at 2^17..2^21. The line is
+//    therefore 2^18 (kTwoPassFrom). An output that overlaps the input other than exactly
+//    in place keeps the single pass there, in which a tile writes only after all tiles
+//    before it have been read.
 //  - Wave form: one cooperative launch walks the input in waves of 2^24 values (64 MB,
 //    half of L2). Per wave every CTA sums its chunk, the grid meets at a counting
 //    barrier, and every CTA scans its chunk while most of it is still in L2. Each CTA
@@ -82,7 +89,8 @@ __global__ void __launch_bounds__(kScanBlock, 6)
 //    re-read saves. Launch-shape variants 11-13 run the scan in waves of 2^22, 2^23 and
 //    2^24 values.
 constexpr int kChunkCtasPerSm = 4;
-constexpr long long kTwoPassMinN = 1LL << 22;
+constexpr long long kTwoPassFrom = 1LL << 18;  // two kernels by default
+constexpr long long kTwoPassMinN = 1LL << 22;  // whatever the overlap; the wave variants
 constexpr long long kWaveValues = 1LL << 24;  // 64 MB of int32 per wave
 constexpr long long kWaveMinN = 1LL << 24;    // compaction: the wave form from here on
 constexpr unsigned long long kWaveBarrierTimeoutNs = 10ull * 1000000000ull;
@@ -987,6 +995,13 @@ hhs_status launch_split_list(const int32_t* list_in, int n, const double* ts, do
 
 unsigned* scan_workspace_error_word(void* ws) { return &static_cast<ScanHeader*>(ws)->error; }
 
+// Whether n values at a and n values at b share memory.
+static bool overlap(const int32_t* a, const int32_t* b, int64_t n) {
+    const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    const uintptr_t bytes = (uintptr_t)n * sizeof(int32_t);
+    return x < y ? y - x < bytes : x - y < bytes;
+}
+
 extern "C" size_t hhs_scan_workspace_size(int64_t n) {
     return scan_workspace_bytes(n, kScanMinTile);
 }
@@ -1015,7 +1030,10 @@ extern "C" hhs_status hhs_scan_exclusive_i32(const int32_t* d_in, int32_t* d_out
                                                          workspace_bytes, nullptr, nullptr, s);
         if (st != kStreamUnavailable) return st;
     }
-    if ((variant == 0 || (variant >= 11 && variant <= 13)) && n >= kTwoPassMinN) {
+    const bool two_kernels = variant == 0 && n >= kTwoPassFrom &&
+                             (d_in == d_out || !overlap(d_in, d_out, n));
+    if (two_kernels ||
+        ((variant == 0 || (variant >= 11 && variant <= 13)) && n >= kTwoPassMinN)) {
         // the chunk sums are written before they are read: only the header is cleared.
         // Default: the two-kernel form; variants 11-13: waves of 2^22, 2^23, 2^24 values.
         const long long wave = variant == 11   ? (1LL << 22)
@@ -1080,7 +1098,10 @@ extern "C" hhs_status hhs_compact_flags_i32(const int32_t* d_flags, int32_t* d_s
                                                         d_count, s);
         if (st != kStreamUnavailable) return st;
     }
-    if (n >= kTwoPassMinN) {
+    // an index list over the flags is filled behind the reads by the single pass only
+    const bool apart = !overlap(d_flags, d_idx, n) &&
+                       (!d_scan || d_scan == d_flags || !overlap(d_flags, d_scan, n));
+    if (n >= kTwoPassMinN || (n >= kTwoPassFrom && apart)) {
         auto* agg = reinterpret_cast<unsigned*>(status);
         const size_t words =
             (scan_workspace_bytes(n, kScanMinTile) - sizeof(ScanHeader)) / sizeof(unsigned);
