@@ -410,77 +410,41 @@ __device__ __forceinline__ int block_sum(int v, Smem& sm) {
 }
 
 // ---------------------------------------------------------------- timestep units
-template <int PREC>
+// FP64: the exact minimum of one block of kEB rows over the columns [j0, j1)
 __device__ void ts_unit(const EParams& E, const int32_t* S, int n, int ib, int j0, int j1,
-                        double* out64, float* out32, Smem& sm) {
+                        double* out, Smem& sm) {
     const int i = ib * kEB + threadIdx.x;
     const bool act = i < n;
     const int gi = act ? list_at(S, i) : 0;
     const SoA& P = E.P;
-    if (PREC == HHS_PREC_FP64) {
-        double xi = 0, yi = 0, zi = 0, vxi = 0, vyi = 0, vzi = 0, mi = 0;
-        if (act) {
-            xi = P.x[gi]; yi = P.y[gi]; zi = P.z[gi];
-            vxi = P.vx[gi]; vyi = P.vy[gi]; vzi = P.vz[gi]; mi = P.m[gi];
-        }
-        double minval = 1.e30;
-        for (int t0 = j0; t0 < j1; t0 += kEB) {
-            const int tl = min(kEB, j1 - t0);
-            __syncthreads();
-            if ((int)threadIdx.x < tl) {
-                const int gj = list_at(S, t0 + threadIdx.x);
-                sm.u.tsd.x[threadIdx.x] = P.x[gj]; sm.u.tsd.y[threadIdx.x] = P.y[gj];
-                sm.u.tsd.z[threadIdx.x] = P.z[gj]; sm.u.tsd.vx[threadIdx.x] = P.vx[gj];
-                sm.u.tsd.vy[threadIdx.x] = P.vy[gj]; sm.u.tsd.vz[threadIdx.x] = P.vz[gj];
-                sm.u.tsd.m[threadIdx.x] = P.m[gj];
-            }
-            __syncthreads();
-            if (act) {
-                for (int jl = 0; jl < tl; jl++) {
-                    if (t0 + jl == i) continue;
-                    ts_pair_fp64(f64_sub(xi, sm.u.tsd.x[jl]), f64_sub(yi, sm.u.tsd.y[jl]),
-                                 f64_sub(zi, sm.u.tsd.z[jl]), f64_sub(vxi, sm.u.tsd.vx[jl]),
-                                 f64_sub(vyi, sm.u.tsd.vy[jl]), f64_sub(vzi, sm.u.tsd.vz[jl]),
-                                 mi, sm.u.tsd.m[jl], E.eta, E.eta_s2, minval);
-                }
-            }
-        }
-        if (act) out64[i] = minval;
-    } else {
-        DS xi{0, 0}, yi{0, 0}, zi{0, 0};
-        float vxi = 0, vyi = 0, vzi = 0, mi = 0;
-        if (act) {
-            xi = ds_split(P.x[gi]); yi = ds_split(P.y[gi]); zi = ds_split(P.z[gi]);
-            vxi = (float)P.vx[gi]; vyi = (float)P.vy[gi]; vzi = (float)P.vz[gi];
-            mi = (float)P.m[gi];
-        }
-        float maxrate = 0.0f;
-        for (int t0 = j0; t0 < j1; t0 += kEB) {
-            const int tl = min(kEB, j1 - t0);
-            __syncthreads();
-            if ((int)threadIdx.x < tl) {
-                const int gj = list_at(S, t0 + threadIdx.x);
-                const DS a = ds_split(P.x[gj]), b = ds_split(P.y[gj]), c = ds_split(P.z[gj]);
-                sm.u.tsm.A[threadIdx.x] = make_float4(a.hi, b.hi, c.hi, (float)P.m[gj]);
-                sm.u.tsm.B[threadIdx.x] = make_float4(a.lo, b.lo, c.lo, 0.0f);
-                sm.u.tsm.V[threadIdx.x] =
-                    make_float4((float)P.vx[gj], (float)P.vy[gj], (float)P.vz[gj], 0.0f);
-            }
-            __syncthreads();
-            if (act) {
-                for (int jl = 0; jl < tl; jl++) {
-                    if (t0 + jl == i) continue;
-                    const float4 A = sm.u.tsm.A[jl], B = sm.u.tsm.B[jl], V = sm.u.tsm.V[jl];
-                    const float r = ts_pair_rate_mixed(
-                        ds_diff(xi.hi, xi.lo, A.x, B.x), ds_diff(yi.hi, yi.lo, A.y, B.y),
-                        ds_diff(zi.hi, zi.lo, A.z, B.z), vxi - V.x, vyi - V.y, vzi - V.z,
-                        mi + A.w, E.inv_eta_s2, E.inv_eta);
-                    maxrate = fmaxf(maxrate, r);
-                }
-            }
-        }
-        if (act) out32[i] = maxrate;
+    double xi = 0, yi = 0, zi = 0, vxi = 0, vyi = 0, vzi = 0, mi = 0;
+    if (act) {
+        xi = P.x[gi]; yi = P.y[gi]; zi = P.z[gi];
+        vxi = P.vx[gi]; vyi = P.vy[gi]; vzi = P.vz[gi]; mi = P.m[gi];
     }
+    double minval = 1.e30;
+    for (int t0 = j0; t0 < j1; t0 += kEB) {
+        const int tl = min(kEB, j1 - t0);
+        __syncthreads();
+        if ((int)threadIdx.x < tl) {
+            const int gj = list_at(S, t0 + threadIdx.x);
+            sm.u.tsd.x[threadIdx.x] = P.x[gj]; sm.u.tsd.y[threadIdx.x] = P.y[gj];
+            sm.u.tsd.z[threadIdx.x] = P.z[gj]; sm.u.tsd.vx[threadIdx.x] = P.vx[gj];
+            sm.u.tsd.vy[threadIdx.x] = P.vy[gj]; sm.u.tsd.vz[threadIdx.x] = P.vz[gj];
+            sm.u.tsd.m[threadIdx.x] = P.m[gj];
+        }
+        __syncthreads();
+        if (act) {
+            for (int jl = 0; jl < tl; jl++) {
+                if (t0 + jl == i) continue;
+                ts_pair_fp64(f64_sub(xi, sm.u.tsd.x[jl]), f64_sub(yi, sm.u.tsd.y[jl]),
+                             f64_sub(zi, sm.u.tsd.z[jl]), f64_sub(vxi, sm.u.tsd.vx[jl]),
+                             f64_sub(vyi, sm.u.tsd.vy[jl]), f64_sub(vzi, sm.u.tsd.vz[jl]),
+                             mi, sm.u.tsd.m[jl], E.eta, E.eta_s2, minval);
+            }
+        }
+    }
+    if (act) out[i] = minval;
 }
 
 
@@ -3657,8 +3621,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     for (int u = W.id; u < nsb * nch; u += W.count) {
                         const int ib = u / nch, jc = u % nch;
                         const int j0 = jc * C, j1 = min(n, j0 + C);
-                        ts_unit<PREC>(E, S, n, ib, j0, j1, E.ts_part + (size_t)jc * E.n_max,
-                                      nullptr, sm);
+                        ts_unit(E, S, n, ib, j0, j1, E.ts_part + (size_t)jc * E.n_max, sm);
                     }
                 } else if (PREC == HHS_PREC_FP64) {
                     // blocks of rows over the workers (one CTA, or the cluster's), as many rows
@@ -3947,7 +3910,7 @@ __global__ void __launch_bounds__(kEB, 2)
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
         const int ib = ib_lo + u / nch, jc = u % nch;
         const int j0 = jc * C, j1 = min(n, j0 + C);
-        ts_unit<HHS_PREC_FP64>(E, S, n, ib, j0, j1, E.ts_part + (size_t)jc * E.n_max, nullptr, sm);
+        ts_unit(E, S, n, ib, j0, j1, E.ts_part + (size_t)jc * E.n_max, sm);
     }
 }
 
