@@ -32,6 +32,15 @@ __device__ __forceinline__ void fence_barrier_init() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Orders ordinary (generic proxy) accesses that happen before it -- the calling thread's, and
+// those of threads it has synchronised with -- and bulk copies that happen after it. Barriers
+// and release / acquire pairs alone order the generic proxy only: a copy could read the
+// global records, or land in the shared buffer, from before another CTA's or thread's
+// ordinary stores.
+__device__ __forceinline__ void fence_proxy_async() {
+    asm volatile("fence.proxy.async;" ::: "memory");
+}
+
 // Arrive and add `bytes` to the transaction count of the current phase.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
