@@ -245,12 +245,14 @@ __global__ void __launch_bounds__(32 * kPmWarps, 3)
     const int j1 = (int)((long long)m * (warp + 1) / kPmWarps);
     int j0 = (int)((long long)m * warp / kPmWarps);
     double sx = 0.0, sy = 0.0, sz = 0.0, sm = 0.0;
+    // Past the slice, its last source without mass: a pair of the sink with a place of its own
+    // (the origin, say) could overflow where no source does, and 0 times that is a NaN.
     auto load = [&](int j) {
-        const bool in = j < j1;
-        sx = in ? S.x[j] : 0.0; sy = in ? S.y[j] : 0.0; sz = in ? S.z[j] : 0.0;
-        sm = in ? S.m[j] : 0.0;
+        const int k = min(j, j1 - 1);
+        sx = S.x[k]; sy = S.y[k]; sz = S.z[k];
+        sm = j < j1 ? S.m[k] : 0.0;
     };
-    load(j0 + lane);
+    if (j0 < j1) load(j0 + lane);
     for (; j0 < j1; j0 += 32) {
         __syncwarp();  // the previous sources are read
         {
