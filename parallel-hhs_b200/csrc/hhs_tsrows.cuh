@@ -18,6 +18,13 @@ __device__ __forceinline__ int ts_list_at(const int32_t* list, int i) { return l
 // Each row starts from its exact rates over the first 32 columns. The result is the maximum
 // over all pairs, as if every one had been evaluated.
 //
+// The squares come from dot products, whose rounding grows with |x|^2 and |v|^2, so the test takes
+// positions and velocities from a centre: the medians of some members, which neither a distant
+// origin, a common velocity nor a few outlying members move away from the rest. (The subtraction
+// is one FP64 rounding of the difference itself.) In FP32 from there on: rounded coordinates, their
+// squares and the dot products err by less than 1.2e-6 of |x_i|^2 + |x_j|^2, which shrinking
+// |x|^2 and growing |v|^2 by 4e-6 covers.
+//
 // The test here is for the row alone, with its rate T = 0.99 best: a pair may be left out if
 //     A >= kappa B + C (p_i + p_j) and B >= D (p_i + p_j),  p = |m|^(2/3),
 // A = |x_i - x_j|^2, B = |v_i - v_j|^2, C = (2 / (eta beta T)^2)^(2/3), D = (1 / (2 (1 - alpha)
@@ -84,6 +91,11 @@ __device__ __forceinline__ double ts_of_key(unsigned long long key) {
     return t < kHuge ? t : kHuge;
 }
 
+// 1.01 |m|^(2/3); the hardware's base-2 functions are within 2e-5 over the range of a float
+__device__ __forceinline__ float ts_mass_term(double m) {
+    return 1.01f * exp2f(0.66666667f * __log2f((float)fabs(m)));
+}
+
 template <int PREC>
 __device__ __forceinline__ TsRowTest ts_row_test(const TsState& q, unsigned long long key,
                                                  const TsArgs& A) {
@@ -95,7 +107,7 @@ __device__ __forceinline__ TsRowTest ts_row_test(const TsState& q, unsigned long
     const float k = e / (kTsAlpha * T), f = eta * beta * T, c = cbrtf(2.01f / (f * f));
     const float kappa = 1.01f * k * k, C = 1.02f * c * c;
     const float h = 0.5f / ((1.0f - kTsAlpha) * T * C), D = 1.02f * h * h;
-    const float pm = cbrtf((float)fabs(q.m)), p = 1.01f * pm * pm;
+    const float p = ts_mass_term(q.m);
     const float W = (float)(r2 * (1.0 - 4e-6)), U = (float)(v2 * (1.0 + 4e-6));
     // without a usable rate (or for eta beyond the test's range) every pair passes
     const bool ok = A.eta <= 1.0 && rate > 1e-12 && rate < 1e12 && r2 < 1e24 && v2 < 1e24 &&
@@ -115,10 +127,38 @@ __device__ __forceinline__ TsRowTest ts_row_test(const TsState& q, unsigned long
     return r;
 }
 
+// The centre: medians (upper ones) over 8 members spread over the n. ts_centre_sample is the calling
+// lane's member (lane modulo 8) in component 0..5 = x, y, z, vx, vy, vz; ts_median the median of a
+// warp's samples in all lanes, NaNs left out; 0 if they are half of them.
+__device__ __forceinline__ double ts_centre_sample(const SoA& P, const int32_t* list, int n,
+                                                   int component) {
+    const double* a = component == 0 ? P.x : component == 1 ? P.y : component == 2 ? P.z
+                      : component == 3 ? P.vx : component == 4 ? P.vy : P.vz;
+    return a[ts_list_at(list, (int)((long long)(threadIdx.x & 7) * n >> 3))];
+}
+__device__ __forceinline__ double ts_median(double v) {
+    const int q = threadIdx.x & 7;
+    const float f = (float)v;  // ranked in FP32: a centre need not be exact
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const float o = __shfl_sync(HHS_FULL_MASK, f, j);
+        rank += o < f || (o == f && j < q) ? 1 : 0;
+    }
+    const unsigned mid = __ballot_sync(HHS_FULL_MASK, rank == 4 && f == f);
+    const double c = __shfl_sync(HHS_FULL_MASK, v, mid ? __ffs(mid) - 1 : 0);
+    return mid ? c : 0.0;
+}
+__device__ __forceinline__ TsState ts_from(const TsState& q, const double* centre) {
+    return TsState{q.x - centre[0], q.y - centre[1], q.z - centre[2], q.vx - centre[3],
+                   q.vy - centre[4], q.vz - centre[5], q.m};
+}
+
 struct TsRows {  // shared memory of ts_rows
     TsState row[kTsMaxRows];
     TsRowTest test[kTsMaxRows];
     unsigned long long best[kTsMaxRows];
+    double centre[6];
     int2 hit[kTsCap];  // (row, column)
     unsigned cnt;
 };
@@ -132,6 +172,7 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
     if (tid < nrow) sm.row[tid] = ts_load(P, ts_list_at(list, i0 + tid));
     if (tid < kTsMaxRows) sm.best[tid] = 0ull;
     if (tid == 0) sm.cnt = 0u;
+    const double sample = tid < 6 * 32 ? ts_centre_sample(P, list, n, tid >> 5) : 0.0;
     __syncthreads();
     for (int k = tid; k < nrow * kTsSeed; k += kTsThreads) {
         const int r = k / kTsSeed, j = k % kTsSeed;
@@ -140,8 +181,11 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
             if (q > sm.best[r]) atomicMax(&sm.best[r], q);
         }
     }
+    __syncwarp();
+    const double median = ts_median(sample);
+    if (tid < 6 * 32 && (tid & 31) == 0) sm.centre[tid >> 5] = median;
     __syncthreads();
-    if (tid < nrow) sm.test[tid] = ts_row_test<PREC>(sm.row[tid], sm.best[tid], A);
+    if (tid < nrow) sm.test[tid] = ts_row_test<PREC>(ts_from(sm.row[tid], sm.centre), sm.best[tid], A);
     __syncthreads();
     unsigned held = 0u;
     for (int t0 = 0; t0 < n; t0 += kTsCols) {
@@ -149,25 +193,27 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
         float2 X, Y, Z, VX, VY, VZ, W, U, p;
 #pragma unroll
         for (int c = 0; c < 2; c++) {
-            const TsState q = j0 + c < n ? ts_load(P, ts_list_at(list, j0 + c))
-                                         : TsState{0, 0, 0, 0, 0, 0, 0};
-            const double r2 = q.x * q.x + q.y * q.y + q.z * q.z,
-                         v2 = q.vx * q.vx + q.vy * q.vy + q.vz * q.vz;
-            const float pm = cbrtf((float)fabs(q.m)), pc = 1.01f * pm * pm;
-            const bool ok = r2 < 1e24 && v2 < 1e24 && pc < 1e20f;  // else it passes every test
+            const TsState q = j0 + c < n
+                                  ? ts_from(ts_load(P, ts_list_at(list, j0 + c)), sm.centre)
+                                  : TsState{0, 0, 0, 0, 0, 0, 0};
+            const float x = (float)q.x, y = (float)q.y, z = (float)q.z;
+            const float vx = (float)q.vx, vy = (float)q.vy, vz = (float)q.vz;
+            const float r2 = x * x + y * y + z * z, v2 = vx * vx + vy * vy + vz * vz;
+            const float pc = ts_mass_term(q.m);
+            const bool ok = r2 < 1e24f && v2 < 1e24f && pc < 1e20f;  // else it passes every test
             auto put = [&](float2& v, float f) {
                 if (c) v.y = f;
                 else v.x = f;
             };
-            put(X, ok ? (float)q.x : 0.0f);
-            put(Y, ok ? (float)q.y : 0.0f);
-            put(Z, ok ? (float)q.z : 0.0f);
-            put(VX, ok ? (float)q.vx : 0.0f);
-            put(VY, ok ? (float)q.vy : 0.0f);
-            put(VZ, ok ? (float)q.vz : 0.0f);
+            put(X, ok ? x : 0.0f);
+            put(Y, ok ? y : 0.0f);
+            put(Z, ok ? z : 0.0f);
+            put(VX, ok ? vx : 0.0f);
+            put(VY, ok ? vy : 0.0f);
+            put(VZ, ok ? vz : 0.0f);
             put(p, ok ? pc : 0.0f);
-            put(W, ok ? (float)(r2 * (1.0 - 4e-6)) : -kTsAll);
-            put(U, ok ? (float)(v2 * (1.0 + 4e-6)) : 0.0f);
+            put(W, ok ? r2 * (1.0f - 4e-6f) : -kTsAll);
+            put(U, ok ? v2 * (1.0f + 4e-6f) : 0.0f);
         }
         for (int r = 0; r < nrow; r++) {
             __syncwarp();  // lanes that listed pairs rejoin the others here
@@ -212,7 +258,7 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
         }
         __syncthreads();
         if (tid == 0) sm.cnt = 0u;
-        if (tid < nrow) sm.test[tid] = ts_row_test<PREC>(sm.row[tid], sm.best[tid], A);
+        if (tid < nrow) sm.test[tid] = ts_row_test<PREC>(ts_from(sm.row[tid], sm.centre), sm.best[tid], A);
         __syncthreads();
         held = 0u;
     }
