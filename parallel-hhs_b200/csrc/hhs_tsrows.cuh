@@ -41,6 +41,7 @@ constexpr int kTsSeed = 32;              // columns that every row evaluates fir
 constexpr int kTsCap = 2048;             // pairs listed at a time
 constexpr unsigned kTsBatch = 64;        // listed pairs that are worth evaluating together
 constexpr int kTsMaxRows = 32;
+constexpr int kTsDense = 7;
 constexpr float kTsAlpha = 0.9f;
 constexpr float kTsAll = 1.0e38f;
 
@@ -154,14 +155,57 @@ __device__ __forceinline__ TsState ts_from(const TsState& q, const double* centr
                    q.vy - centre[4], q.vz - centre[5], q.m};
 }
 
+// A row of the mixed rates: the negated particle, each value in both lanes when used.
+struct TsSink {
+    float nxh, nyh, nzh, nxl, nyl, nzl, nvx, nvy, nvz, m;
+};
+__device__ __forceinline__ TsSink ts_sink(const TsState& q) {
+    const DS x = ds_split(q.x), y = ds_split(q.y), z = ds_split(q.z);
+    return TsSink{-x.hi, -y.hi, -z.hi, -x.lo, -y.lo, -z.lo,
+                  -(float)q.vx, -(float)q.vy, -(float)q.vz, (float)q.m};
+}
+
 struct TsRows {  // shared memory of ts_rows
     TsState row[kTsMaxRows];
     TsRowTest test[kTsMaxRows];
     unsigned long long best[kTsMaxRows];
     double centre[6];
+    TsSink sink[kTsMaxRows];  // mixed
     int2 hit[kTsCap];  // (row, column)
     unsigned cnt;
 };
+
+// Every rate of the rows against the columns t0 .. t0 + kTsCols - 1 in mixed precision, two columns
+// a thread, without a list.
+__device__ __forceinline__ void ts_dense_tile(const SoA& P, const int32_t* list, int n, int i0,
+                                              int nrow, int t0, const TsArgs& A, TsRows& sm) {
+    const int j0 = t0 + 2 * (int)threadIdx.x;
+    float2 xh, yh, zh, xl, yl, zl, vx, vy, vz, m;
+    {
+        // (past the end: the last particle again, left out below)
+        const TsState a = ts_load(P, ts_list_at(list, min(j0, n - 1))),
+                      b = ts_load(P, ts_list_at(list, min(j0 + 1, n - 1)));
+        const DS ax = ds_split(a.x), ay = ds_split(a.y), az = ds_split(a.z);
+        const DS bx = ds_split(b.x), by = ds_split(b.y), bz = ds_split(b.z);
+        xh = make_float2(ax.hi, bx.hi); yh = make_float2(ay.hi, by.hi); zh = make_float2(az.hi, bz.hi);
+        xl = make_float2(ax.lo, bx.lo); yl = make_float2(ay.lo, by.lo); zl = make_float2(az.lo, bz.lo);
+        vx = make_float2((float)a.vx, (float)b.vx); vy = make_float2((float)a.vy, (float)b.vy);
+        vz = make_float2((float)a.vz, (float)b.vz); m = make_float2((float)a.m, (float)b.m);
+    }
+    for (int r = 0; r < nrow; r++) {
+        const TsSink q = sm.sink[r];
+        const TsSink2 s{f2dup(q.nxh), f2dup(q.nyh), f2dup(q.nzh), f2dup(q.nxl), f2dup(q.nyl),
+                        f2dup(q.nzl), f2dup(q.nvx), f2dup(q.nvy), f2dup(q.nvz), f2dup(q.m)};
+        const float2 rate = ts_pair_rate_mixed2(xh, yh, zh, xl, yl, zl, vx, vy, vz, m, s,
+                                                A.inv_eta_s2, A.inv_eta);
+        const int i = i0 + r;
+        const float best = fmaxf(fmaxf(j0 < n && j0 != i ? rate.x : 0.0f,
+                                       j0 + 1 < n && j0 + 1 != i ? rate.y : 0.0f), 0.0f);
+        const unsigned key = __reduce_max_sync(HHS_FULL_MASK, __float_as_uint(best));
+        if ((threadIdx.x & 31) == 0 && key > *(volatile unsigned long long*)&sm.best[r])
+            atomicMax(&sm.best[r], (unsigned long long)key);
+    }
+}
 
 // The keys of rows i0 .. i0 + nrow - 1 (at most kTsMaxRows) of the n particles of `list` into
 // sm.best. Called by all kTsThreads threads of the CTA; ends with a CTA barrier.
@@ -169,7 +213,10 @@ template <int PREC>
 __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n, int i0, int nrow,
                                         const TsArgs& A, TsRows& sm) {
     const int tid = threadIdx.x;
-    if (tid < nrow) sm.row[tid] = ts_load(P, ts_list_at(list, i0 + tid));
+    if (tid < nrow) {
+        sm.row[tid] = ts_load(P, ts_list_at(list, i0 + tid));
+        if (PREC == HHS_PREC_MIXED) sm.sink[tid] = ts_sink(sm.row[tid]);
+    }
     if (tid < kTsMaxRows) sm.best[tid] = 0ull;
     if (tid == 0) sm.cnt = 0u;
     const double sample = tid < 6 * 32 ? ts_centre_sample(P, list, n, tid >> 5) : 0.0;
@@ -188,7 +235,13 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
     if (tid < nrow) sm.test[tid] = ts_row_test<PREC>(ts_from(sm.row[tid], sm.centre), sm.best[tid], A);
     __syncthreads();
     unsigned held = 0u;
+    int dense = 0;  // tiles to come that are not tested
     for (int t0 = 0; t0 < n; t0 += kTsCols) {
+        if (PREC == HHS_PREC_MIXED && dense > 0) {
+            dense--;
+            ts_dense_tile(P, list, n, i0, nrow, t0, A, sm);
+            continue;
+        }
         const int j0 = t0 + 2 * tid;
         float2 X, Y, Z, VX, VY, VZ, W, U, p;
 #pragma unroll
@@ -245,9 +298,15 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
             continue;
         }
         // the listed pairs; if the list overflowed, those of earlier tiles and every pair of
-        // this one
+        // this one, in mixed precision also of the next kTsDense tiles without a test. (A listed
+        // pair takes as long as five in dense tiles: 16384 mixed, all pairs pass, 3104 us with lists, 755)
         const bool all = cnt > kTsCap;
-        const int listed = (int)(all ? held : cnt), total = listed + (all ? nrow * kTsCols : 0);
+        const int listed = (int)(all ? held : cnt),
+                  total = listed + (all && PREC == HHS_PREC_FP64 ? nrow * kTsCols : 0);
+        if (PREC == HHS_PREC_MIXED && all) {
+            ts_dense_tile(P, list, n, i0, nrow, t0, A, sm);
+            dense = kTsDense;
+        }
         for (int k = tid; k < total; k += kTsThreads) {
             const int2 h = k < listed ? sm.hit[k]
                                       : make_int2((k - listed) / kTsCols, t0 + (k - listed) % kTsCols);
@@ -262,6 +321,7 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
         __syncthreads();
         held = 0u;
     }
+    if (PREC == HHS_PREC_MIXED) __syncthreads();  // the last tile may have been a dense one
 }
 
 }  // namespace hhs

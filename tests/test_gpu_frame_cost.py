@@ -41,3 +41,41 @@ def test_timesteps_call(cuda, hhs, n, prec):
     plain = ms(0.0, 0.0)
     assert ms(1000.0, 0.0) < 1.5 * plain + 0.01
     assert ms(0.0, 200.0) < 1.5 * plain + 0.01
+
+
+def _pair_of_clusters(hhs, n, distance):
+    s = hhs.plummer(n, 5)
+    s["x"][n // 2:] += distance
+    return s
+
+
+@pytest.mark.parametrize("kind,n", [("eta", 16384), ("clusters", 16384), ("eta", 4097)])
+def test_timesteps_call_that_the_filter_does_not_help(cuda, hhs, kind, n):
+    """Every pair passes (the test's range ends at eta = 1), or half of them do (two clusters far
+    apart): the evaluation of every pair without a test takes 3 times the filtered call's."""
+    def ms(s, eta):
+        d = hhs.ParticleSystem(n)
+        d.upload(s)
+        ctx = hhs.Context(n, 8, eta)
+        return _least_ms(cuda, lambda: hhs.timesteps(ctx, d, n, hhs.PREC_MIXED), lambda: None)
+
+    plain = ms(hhs.plummer(n, 5), 0.03)
+    other = ms(hhs.plummer(n, 5), 1.5) if kind == "eta" else ms(_pair_of_clusters(hhs, n, 1e3), 0.03)
+    assert other < 4.5 * plain
+
+
+@pytest.mark.parametrize("n", [3, 511, 513, 4097, 9999])
+def test_dense_tiles(cuda, hhs, oracle, n):
+    """Two clusters far apart, member by member: tiles of which half the pairs pass. Positions on a
+    grid of 2^-20 lengths are exact in double-single form at a distance of 2^12, so the bound of
+    the mixed timesteps holds; eta beyond the test's range passes all."""
+    s = hhs.plummer(n, 7)
+    for k in ("x", "y", "z"):
+        s[k] = np.round(s[k] * 2.0 ** 20) / 2.0 ** 20
+    s["x"][1::2] += 4096.0
+    for eta in (0.03, 1.5):
+        d = hhs.ParticleSystem(n)
+        d.upload(s)
+        hhs.timesteps(hhs.Context(n, 8, eta), d, n, hhs.PREC_MIXED)
+        ref = oracle.timesteps(s, eta)
+        assert np.all(np.abs(d.download()["ts"] - ref) <= 2e-6 * ref)
