@@ -69,6 +69,7 @@ struct EngineState {
     unsigned m_max;       // largest |mass| of the launch's system (FP32 bits, cleared likewise)
     unsigned pad[2];
     unsigned kick_ctr[2][kMaxLevels];  // dynamic work counters of each level's kick units
+    double centre[6];  // of the fast set whose filter records the next kick reduction writes
     unsigned long long prof_ns[8];
     unsigned long long prof_cnt[8];
     double prof_pairs[8];
@@ -186,6 +187,7 @@ struct __align__(16) Smem {
     unsigned tf_cnt;              // filtered timestep: passing pairs, of which
     int tf_n;                     // tf_n are listed, and the first unit that overflowed the
     long long tf_ov;              // list (-1: none)
+    double centre[6];             // of the node whose filter records this CTA writes
     unsigned kphase;              // parity of the next phase of kbar
     unsigned tphase;              // parities of the next phases of tbar[0], tbar[1]
     __align__(8) uint64_t kbar;   // completion barrier of the kick's source-tile copies
@@ -811,7 +813,11 @@ __device__ void ts_sym_tiles(const EParams& E, int n, int cw, long long u0, long
 // Both squares come from dot products, A = |x_i|^2 + |x_j|^2 - 2 x_i x_j: 9 packed operations
 // for two pairs, where their rates take about a hundred instructions. Rounding (below 1.5e-6 of
 // |x_i|^2 + |x_j|^2) is covered by shrinking the |x|^2 and growing the |v|^2 by 4e-6, which
-// keeps the computed A below and B above the true ones, and by a margin in b.
+// keeps the computed A below and B above the true ones, and by a margin in b. So that these
+// margins are those of the node's own extent, x and v are taken from a centre, the medians of
+// some members (as in hhs_tsrows.cuh): one FP64 rounding of the differences. The kick phase
+// before a kick reduction takes it from the fast set (its last CTA, about a microsecond of that
+// CTA's), since the reduction itself changes the velocities.
 // Measured: the timestep phases of an N=65536 step (Salpeter masses) 123.0 -> 41 ms, 16384 4.10 ->
 // 2.24 (FP64: 40.7 -> 2.6); a calc of 64678 members 1.21 ms, 1.7e12 unordered pairs/s. What
 // bounds it: the FMA pipe (half busy) and, below about 6000 members, the latency of the tiles.
@@ -831,10 +837,18 @@ __device__ __forceinline__ double tf_bound(const EParams& E, int i, int g, bool 
     return t > 1e-12 && t < 1e12 ? t : 0.0;
 }
 
-// Member i for the filter, bound as tf_bound gives it: component i & 1 of its entry.
-__device__ __forceinline__ void tf_put(const EParams& E, int i, double x, double y, double z,
-                                       double vx, double vy, double vz, double mass,
-                                       double bound) {
+// Component `warp` of the centre of n members of S, by the calling CTA's first six warps.
+__device__ __forceinline__ void tf_centre(const EParams& E, const int32_t* S, int n, double* out) {
+    const int warp = threadIdx.x >> 5;
+    if (warp >= 6) return;
+    const double c = ts_median(ts_centre_sample(E.P, S, n, warp));
+    if ((threadIdx.x & 31) == 0) out[warp] = c;
+}
+
+// Member i (its state q from the node's centre) for the filter, bound as tf_bound gives it:
+// component i & 1 of its entry.
+__device__ __forceinline__ void tf_put(const EParams& E, int i, const TsState& q0, double bound) {
+    const double x = q0.x, y = q0.y, z = q0.z, vx = q0.vx, vy = q0.vy, vz = q0.vz, mass = q0.m;
     const double r2 = x * x + y * y + z * z, v2 = vx * vx + vy * vy + vz * vz;
     const float T = 0.99f * (float)bound, eta = (float)E.eta;
     const float M = (float)fabs(mass) + __uint_as_float(__ldcg(&E.st->m_max));
@@ -1102,12 +1116,14 @@ __device__ void pack_ts(const EParams& E, const int32_t* S, int n, const Workers
 
 // The same for the filter.
 template <int PREC>
-__device__ void pack_tf(const EParams& E, const int32_t* S, int n, bool top, const Workers& W) {
+__device__ void pack_tf(const EParams& E, const int32_t* S, int n, bool top, const Workers& W,
+                        Smem& sm) {
     const SoA& P = E.P;
+    tf_centre(E, S, n, sm.centre);
+    __syncthreads();
     for (int i = W.id * kEB + (int)threadIdx.x; i < n; i += W.count * kEB) {
         const int g = list_at(S, i);
-        tf_put(E, i, P.x[g], P.y[g], P.z[g], P.vx[g], P.vy[g], P.vz[g], P.m[g],
-               tf_bound<PREC>(E, i, g, top));
+        tf_put(E, i, ts_from(ts_load(P, g), sm.centre), tf_bound<PREC>(E, i, g, top));
     }
 }
 
@@ -2318,6 +2334,15 @@ __device__ void split_phase(const EParams& E, const int32_t* S, int n, double dt
     }
 }
 
+// Particle g with its new velocity v, from the centre that the kick phase left.
+__device__ __forceinline__ TsState tf_state(const EParams& E, int g, const double* v) {
+    const SoA& P = E.P;
+    double c[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) c[k] = __ldcg(&E.st->centre[k]);
+    return ts_from(TsState{P.x[g], P.y[g], P.z[g], v[0], v[1], v[2], P.m[g]}, c);
+}
+
 // Sum of the per-chunk partial accelerations, v += a*dt, and for slow sinks both half
 // drifts. Mixed: one thread per (sink, component) adds its chunks with eight independent
 // loads in flight, so the reduction of a node spreads over the whole grid; FP64: one
@@ -2349,8 +2374,7 @@ __device__ void kick_reduce_phase(const EParams& E, const int32_t* F, const int3
             }
             P.vx[g] = v1[0]; P.vy[g] = v1[1]; P.vz[g] = v1[2];
             if (FILTER && !slow && E.filter && W.mode == kModeGrid)
-                tf_put(E, s, P.x[g], P.y[g], P.z[g], v1[0], v1[1], v1[2], P.m[g],
-                       tf_bound<PREC>(E, s, g, false));
+                tf_put(E, s, tf_state(E, g, v1), tf_bound<PREC>(E, s, g, false));
             if (slow) {
                 P.x[g] = f64_add(f64_add(P.x[g], f64_mul(v0[0], h)), f64_mul(v1[0], h));
                 P.y[g] = f64_add(f64_add(P.y[g], f64_mul(v0[1], h)), f64_mul(v1[1], h));
@@ -2401,8 +2425,7 @@ __device__ void kick_reduce_phase(const EParams& E, const int32_t* F, const int3
                 if (!slow && E.tq && W.mode == kModeGrid) {
                     // the fast set's next pass recomputes its timesteps from these records
                     if (FILTER && E.filter)
-                        tf_put(E, s2, P.x[g], P.y[g], P.z[g], v1[0], v1[1], v1[2], P.m[g],
-                               tf_bound<PREC>(E, s2, g, false));
+                        tf_put(E, s2, tf_state(E, g, v1), tf_bound<PREC>(E, s2, g, false));
                     else
                         tq_put(E, s2, P.x[g], P.y[g], P.z[g], P.m[g], v1[0], v1[1], v1[2]);
                 }
@@ -3522,6 +3545,13 @@ __device__ __forceinline__ bool kick_overlaps(const EParams& E, int lvl, const W
            ld_volatile_i32(&E.counts[lvl].n_slow) > 0;
 }
 
+// Nodes of at most so many members run with their subtree from shared memory.
+template <int PREC, int MODE>
+__device__ __forceinline__ int mid_limit(const EParams& E) {
+    const int m = min(E.mid_n, kMid);
+    return PREC == HHS_PREC_FP64 && MODE == kModeGrid ? min(m, kMidFp64) : m;
+}
+
 // ---------------------------------------------------------------- the recursion
 // Walks the HOLD recursion from `top` (whose subsystem is already defined by the
 // counts/lists above it). Grid and cluster modes delegate nodes with n <= small_n,
@@ -3545,8 +3575,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 if (threadIdx.x == 0) atomicOr(E.err, HHS_ERRBIT_DEPTH);
                 return false;
             }
-            if (n <= (PREC == HHS_PREC_FP64 && MODE == kModeGrid ? min(E.mid_n, kMidFp64) : E.mid_n) &&
-                n <= kMid) {
+            if (n <= mid_limit<PREC, MODE>(E)) {
                 // the whole subtree from shared memory: on the grid's first cluster (or
                 // CTA 0), on this hardware cluster, or on this CTA alone
                 if constexpr (MODE == kModeGrid) {
@@ -3620,7 +3649,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     }
                     if (FILTER && filtered) {
                         if (pack) {
-                            pack_tf<PREC>(E, S, n, top_node, W);
+                            pack_tf<PREC>(E, S, n, top_node, W, sm);
                             if (!phase_barrier(E, sm, W)) return false;
                         }
                         const int rbn = tf_rows(n), cw = tf_tile_width(n, rbn, W.count);
@@ -3698,6 +3727,9 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 const int C = (ntot + nch - 1) / nch;
                 const int nsb = (ntot + blk - 1) / blk;
                 const double h = dt * 0.5;
+                if (FILTER && MODE == kModeGrid && E.filter && nf > mid_limit<PREC, MODE>(E) &&
+                    W.id == W.count - 1)
+                    tf_centre(E, F, nf, E.st->centre);  // for this node's kick reduction
                 // blocks of fast sinks only need the slow-source chunks: the work units
                 // are the first nfb blocks x jcs chunks, then the other blocks x nch
                 const int nfb = nf / blk;

@@ -79,3 +79,32 @@ def test_dense_tiles(cuda, hhs, oracle, n):
         hhs.timesteps(hhs.Context(n, 8, eta), d, n, hhs.PREC_MIXED)
         ref = oracle.timesteps(s, eta)
         assert np.all(np.abs(d.download()["ts"] - ref) <= 2e-6 * ref)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_step(cuda, hhs, prec):
+    """The phase that computes timesteps in a step, whose pairs the same filter tests. (A shift by
+    a power of two and a rounded start keep the displaced system the same system.)"""
+    n = 9001
+
+    def ms(shift, velocity):
+        s = hhs.plummer(n, 5)
+        for k in ("x", "y", "z", "vx", "vy", "vz"):
+            s[k] = np.round(s[k] * 2.0 ** 32) / 2.0 ** 32
+        s["x"] += shift
+        s["vy"] += velocity
+        d = hhs.ParticleSystem(n)
+        ctx = hhs.Context(n, 64, 0.03)
+        ctx.set_profiling(True)
+        best, before = 1e30, 0.0
+        for _ in range(4):
+            d.upload(s)
+            hhs.hold_step(ctx, d, n, 0.0, 1.0 / 64, True, prec)
+            ctx.check()
+            total = ctx.profile()["timesteps"]["ms"]
+            best, before = min(best, total - before), total
+        return best
+
+    plain = ms(0.0, 0.0)
+    assert ms(1024.0, 0.0) < 1.5 * plain
+    assert ms(0.0, 256.0) < 1.5 * plain
