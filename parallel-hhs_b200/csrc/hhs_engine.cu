@@ -70,6 +70,7 @@ struct EngineState {
     unsigned pad[2];
     unsigned kick_ctr[2][kMaxLevels];  // dynamic work counters of each level's kick units
     double centre[6];  // of the fast set whose filter records the next kick reduction writes
+    unsigned dense;    // nonzero: that set's pairs are evaluated without the filter
     unsigned long long prof_ns[8];
     unsigned long long prof_cnt[8];
     double prof_pairs[8];
@@ -846,8 +847,9 @@ __device__ __forceinline__ void tf_centre(const EParams& E, const int32_t* S, in
 }
 
 // Member i (its state q from the node's centre) for the filter, bound as tf_bound gives it:
-// component i & 1 of its entry.
-__device__ __forceinline__ void tf_put(const EParams& E, int i, const TsState& q0, double bound) {
+// component i & 1 of its entry in `rec`.
+__device__ __forceinline__ void tf_put(const EParams& E, float4* rec, int i, const TsState& q0,
+                                       double bound) {
     const double x = q0.x, y = q0.y, z = q0.z, vx = q0.vx, vy = q0.vy, vz = q0.vz, mass = q0.m;
     const double r2 = x * x + y * y + z * z, v2 = vx * vx + vy * vy + vz * vz;
     const float T = 0.99f * (float)bound, eta = (float)E.eta;
@@ -858,7 +860,7 @@ __device__ __forceinline__ void tf_put(const EParams& E, int i, const TsState& q
     const float h = 0.5f * M / ((1.0f - kTfAlpha) * T * a);
     // false for NaN; without it every pair of the member passes
     const bool ok = r2 < 1e24 && v2 < 1e24 && bound > 0.0 && kappa < 1e24f && a < 1e24f && h < 1e12f;
-    float* q = reinterpret_cast<float*>(E.tf) + 20 * (size_t)(i >> 1) + (i & 1);
+    float* q = reinterpret_cast<float*>(rec) + 20 * (size_t)(i >> 1) + (i & 1);
     q[0] = ok ? (float)x : 0.0f;
     q[2] = ok ? (float)y : 0.0f;
     q[4] = ok ? (float)z : 0.0f;
@@ -1114,16 +1116,48 @@ __device__ void pack_ts(const EParams& E, const int32_t* S, int n, const Workers
     if ((threadIdx.x & 31) == 0 && b) atomicMax(&E.st->m_max, b);
 }
 
-// The same for the filter.
+// Whether so many of the pairs of S would pass the filter that evaluating them all without it is
+// faster: from 2048 pairs of 256 members spread over the n, with the filter's own records and
+// test, by all threads of a CTA (about 2 us of it; every CTA finds the same). sm.centre is set.
+// A pair that passes goes through the list, a gather and two atomics, as long as 40 evaluations in
+// tiles: so it is in systems with one dominating mass (the bounds hold m_i + m_max) and in units
+// that leave the range of the test's FP32 numbers. Milliseconds of timesteps a step, lists / without
+// the filter at all / with this choice: light disk around one mass, 16384 members 1.3 / 0.42 / 0.41,
+// 65536 102.7 / 8.0 / 7.8; 16384 in SI units 68 / 4.2 / 4.1. Elsewhere 0.2% to 0.5% pass.
+// FP64 keeps its lists (an FP64 evaluation of every pair takes longer than the lists do).
+constexpr int kTfDenseFrom = 1024;  // members; smaller nodes' pairs take a few microseconds anyway
+constexpr int kTfDensePass = 50;    // of 2048
+__device__ __forceinline__ bool tf_dense(const EParams& E, const int32_t* S, int n) {
+    Smem& sm = cta_smem();
+    if (n < kTfDenseFrom) return false;
+    const int tid = threadIdx.x;
+    auto& T = sm.u.tf.T[0];
+    static_assert(kEB == kTW, "an entry of the tile for every two threads");
+    const int g = list_at(S, (int)((long long)tid * n / kEB));
+    __syncthreads();
+    tf_put(E, &T[0][0], tid, ts_from(ts_load(E.P, g), sm.centre),
+           tf_bound<HHS_PREC_MIXED>(E, 0, g, false));
+    __syncthreads();
+    const TfRow row = tf_row(&T[0][0], tid);
+    int pass = 0;
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) {
+        float2 v, B;
+        tf_test(T[((tid >> 1) + 1 + 29 * k) & (kEB / 2 - 1)], row, v, B);
+        pass += __syncthreads_count(v.x <= row.c1 || B.x < row.c2);
+        pass += __syncthreads_count(v.y <= row.c1 || B.y < row.c2);
+    }
+    return pass >= kTfDensePass;
+}
+
+// The node's members for the filter, sm.centre taken from them.
 template <int PREC>
 __device__ void pack_tf(const EParams& E, const int32_t* S, int n, bool top, const Workers& W,
                         Smem& sm) {
     const SoA& P = E.P;
-    tf_centre(E, S, n, sm.centre);
-    __syncthreads();
     for (int i = W.id * kEB + (int)threadIdx.x; i < n; i += W.count * kEB) {
         const int g = list_at(S, i);
-        tf_put(E, i, ts_from(ts_load(P, g), sm.centre), tf_bound<PREC>(E, i, g, top));
+        tf_put(E, E.tf, i, ts_from(ts_load(P, g), sm.centre), tf_bound<PREC>(E, i, g, top));
     }
 }
 
@@ -2374,7 +2408,7 @@ __device__ void kick_reduce_phase(const EParams& E, const int32_t* F, const int3
             }
             P.vx[g] = v1[0]; P.vy[g] = v1[1]; P.vz[g] = v1[2];
             if (FILTER && !slow && E.filter && W.mode == kModeGrid)
-                tf_put(E, s, tf_state(E, g, v1), tf_bound<PREC>(E, s, g, false));
+                tf_put(E, E.tf, s, tf_state(E, g, v1), tf_bound<PREC>(E, s, g, false));
             if (slow) {
                 P.x[g] = f64_add(f64_add(P.x[g], f64_mul(v0[0], h)), f64_mul(v1[0], h));
                 P.y[g] = f64_add(f64_add(P.y[g], f64_mul(v0[1], h)), f64_mul(v1[1], h));
@@ -2424,8 +2458,8 @@ __device__ void kick_reduce_phase(const EParams& E, const int32_t* F, const int3
                 P.vx[g] = v1[0]; P.vy[g] = v1[1]; P.vz[g] = v1[2];
                 if (!slow && E.tq && W.mode == kModeGrid) {
                     // the fast set's next pass recomputes its timesteps from these records
-                    if (FILTER && E.filter)
-                        tf_put(E, s2, tf_state(E, g, v1), tf_bound<PREC>(E, s2, g, false));
+                    if (FILTER && E.filter && __ldcg(&E.st->dense) == 0u)
+                        tf_put(E, E.tf, s2, tf_state(E, g, v1), tf_bound<PREC>(E, s2, g, false));
                     else
                         tq_put(E, s2, P.x[g], P.y[g], P.z[g], P.m[g], v1[0], v1[1], v1[2]);
                 }
@@ -3636,7 +3670,13 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     const bool top_node = lvl == top;
                     const bool pack = top_node || ld_volatile_i32(&E.counts[lvl - 1].n_slow) == 0;
                     filtered = filter && (!top_node || PREC == HHS_PREC_FP64);
-                    if (!filter || top_node) {
+                    if (FILTER && filtered && pack) {
+                        tf_centre(E, S, n, sm.centre);
+                        __syncthreads();
+                    }
+                    if (FILTER && filtered && PREC != HHS_PREC_FP64)
+                        filtered = pack ? !tf_dense(E, S, n) : __ldcg(&E.st->dense) == 0u;
+                    if (!filtered || top_node) {
                         if (pack) {
                             pack_ts(E, S, n, W);
                             if (!phase_barrier(E, sm, W)) return false;
@@ -3728,8 +3768,16 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 const int nsb = (ntot + blk - 1) / blk;
                 const double h = dt * 0.5;
                 if (FILTER && MODE == kModeGrid && E.filter && nf > mid_limit<PREC, MODE>(E) &&
-                    W.id == W.count - 1)
-                    tf_centre(E, F, nf, E.st->centre);  // for this node's kick reduction
+                    W.id == W.count - 1) {  // for this node's kick reduction
+                    tf_centre(E, F, nf, sm.centre);
+                    __syncthreads();
+                    if (threadIdx.x < 6) E.st->centre[threadIdx.x] = sm.centre[threadIdx.x];
+                    if (PREC != HHS_PREC_FP64) {
+                        const bool dense = tf_dense(E, F, nf);
+                        if (threadIdx.x == 0) E.st->dense = dense ? 1u : 0u;
+                    }
+                    __syncthreads();
+                }
                 // blocks of fast sinks only need the slow-source chunks: the work units
                 // are the first nfb blocks x jcs chunks, then the other blocks x nch
                 const int nfb = nf / blk;

@@ -108,3 +108,75 @@ def test_step(cuda, hhs, prec):
     plain = ms(0.0, 0.0)
     assert ms(1024.0, 0.0) < 1.5 * plain
     assert ms(0.0, 256.0) < 1.5 * plain
+
+
+def _units(hhs, n):
+    """A cluster in units of 1e-7 of its size and 1e14 of its time."""
+    s = hhs.plummer(n, 5)
+    for k in ("x", "y", "z"):
+        s[k] *= 1e7
+    for k in ("vx", "vy", "vz"):
+        s[k] *= 1e-7
+    s["m"] *= 1e-7
+    return s, 1e14 / 64
+
+
+def _disk(hhs, n):
+    """Light members on nearly circular orbits about one mass."""
+    s = hhs.plummer(n, 5)
+    r = np.random.default_rng(5)
+    a, ph, dv = r.uniform(1, 2, n), r.uniform(0, 2 * np.pi, n), r.normal(size=(3, n)) * 1e-2
+    s["x"][:], s["y"][:], s["z"][:] = a * np.cos(ph), a * np.sin(ph), r.normal(size=n) * 1e-2
+    s["vx"][:] = dv[0] - np.sin(ph) / np.sqrt(a)
+    s["vy"][:] = dv[1] + np.cos(ph) / np.sqrt(a)
+    s["vz"][:] = dv[2]
+    s["m"][:] = 1e-9
+    s["m"][0] = 1.0
+    for k in ("x", "y", "z", "vx", "vy", "vz"):
+        s[k][0] = 0.0
+    return s, 1.0 / 64
+
+
+def _phases(hhs, s, dt, eta, prec):
+    n = len(s["x"])
+    d = hhs.ParticleSystem(n)
+    ctx = hhs.Context(n, 64, eta)
+    ctx.set_profiling(True)
+    best, before = None, None
+    for _ in range(4):
+        d.upload(s)
+        hhs.hold_step(ctx, d, n, 0.0, dt, True, prec)
+        ctx.check()
+        p = {k: v["ms"] for k, v in ctx.profile().items() if isinstance(v, dict) and "ms" in v}
+        now = p if before is None else {k: p[k] - before[k] for k in p}
+        best = now if best is None else {k: min(best[k], now[k]) for k in p}
+        before = p
+    return best
+
+
+def test_step_in_other_units(cuda, hhs):
+    """No pair can be left out where the test's numbers leave their range: the timestep phase then
+    takes the evaluation of every pair, twice the filtered one's time (30 times through lists)."""
+    n = 16384
+    plain = _phases(hhs, hhs.plummer(n, 5), 1.0 / 64, 0.03, hhs.PREC_MIXED)["timesteps"]
+    s, dt = _units(hhs, n)
+    assert _phases(hhs, s, dt, 0.03, hhs.PREC_MIXED)["timesteps"] < 3.0 * plain
+
+
+@pytest.mark.parametrize("n", [6001, 9001, 16384])
+@pytest.mark.parametrize("kind", ["units", "disk"])
+def test_step_without_the_filter_where_it_does_not_help(cuda, hhs, kind, n):
+    """The same bits as the step from equal timesteps, which is never filtered."""
+    s, dt = _units(hhs, n) if kind == "units" else _disk(hhs, n)
+    a, b = hhs.ParticleSystem(n), hhs.ParticleSystem(n)
+    ctx = hhs.Context(n, 64, 0.03)
+    a.upload(s)
+    b.upload(s)
+    hhs.hold_step(ctx, a, n, 0.0, dt, True, hhs.PREC_MIXED)
+    ctx.check()
+    hhs.timesteps(ctx, b, n, hhs.PREC_MIXED)
+    hhs.hold_step(ctx, b, n, 0.0, dt, False, hhs.PREC_MIXED)
+    ctx.check()
+    x, y = a.download(), b.download()
+    for k in ("x", "y", "z", "vx", "vy", "vz", "ts"):
+        assert np.array_equal(x[k], y[k]), k
