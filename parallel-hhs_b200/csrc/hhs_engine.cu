@@ -117,6 +117,7 @@ struct EParams {
     float4* tf;
     unsigned long long* tau_key;  // [n_max] FP64: complement of the least pair timescale's bits
     int filter;      // grid nodes below the top one filter their pairs (tf_row)
+    double tf_guess;  // which guess each rate as at least this times the last one
     int prec_mixed;  // this launch runs the mixed-precision kernels
     int overlap;     // slow-only kick units beside a subtree's first pass (tuning)
     int4* trace;                        // node record {level, n, n_fast, calc} in call order
@@ -823,9 +824,6 @@ __device__ void ts_sym_tiles(const EParams& E, int n, int cw, long long u0, long
 // 2.24 (FP64: 40.7 -> 2.6); a calc of 64678 members 1.21 ms, 1.7e12 unordered pairs/s. What
 // bounds it: the FMA pipe (half busy) and, below about 6000 members, the latency of the tiles.
 constexpr float kTfAlpha = 0.8f;
-// T over the old rate: at 0.7 the larger kappa costs 7% of the calcs at N=16384, at 0.85 a few
-// rows a step are scanned whole (150 us a step)
-constexpr double kTfGuess = 0.8;
 constexpr float kTfAll = 1.0e38f;   // a particle whose pairs all pass
 
 // The lower bound of member i's rate that the filter uses (0: none, every pair passes): from
@@ -834,7 +832,7 @@ template <int PREC>
 __device__ __forceinline__ double tf_bound(const EParams& E, int i, int g, bool top) {
     const double t = PREC == HHS_PREC_FP64 && top
                          ? 0.999 * (double)__uint_as_float(__ldcg(&E.rate_acc[i]))
-                         : kTfGuess / E.P.ts[g];
+                         : E.tf_guess / E.P.ts[g];
     return t > 1e-12 && t < 1e12 ? t : 0.0;
 }
 
@@ -4226,6 +4224,19 @@ std::array<const void*, 5> engine_kernels() {
 // ms of timesteps, at 4099 0.04 of 0.41, and its code costs the subtree solver in the same kernel
 // 3% (registers). FP64 steps always do (a full FP64 evaluation takes ten times as long).
 constexpr int kFilterN = 6000;
+
+// The bound of a rate over the last one. In one timestep a rate changes by a factor of about
+// 1 +- 2 eta at most (it is |dv| / (eta r) or larger), so the guess has to fall with eta: a row
+// whose bound was too high is scanned whole by one warp, and where many are, the scans take
+// longer than all the rest. Milliseconds a step with guesses of 0.8 / 0.5 / 0.3 and without a
+// filter, 16384 mixed: eta 0.03 13.1 / 13.6 / 26.8 / 14.9, 0.15 10.5 / 11.0 / 24.1 / 12.1, 0.2 8.4 /
+// 8.6 / 17.3 / 9.3, 0.25 9.8 / 6.4 / 13.7 / 7.0, 0.5 30.9 / 6.9 / 16.5 / 7.2, 1 22.0 / 8.1 / 5.9 / 4.0;
+// 9001 FP64: 0.03 13.1 / 13.3 / 16.9 / 24.6, 0.2 8.4 / 8.5 / 9.9 / 15.6, 0.5 25.5 / 7.2 / 9.1 / 12.8, 1
+// 18.2 / 7.7 / 5.6 / 7.0. (At 0.03, 0.7 costs 7% of the calcs, 0.85 scans a few rows: 150 us a step.)
+// Rows begin to fail near 0.2 with 0.8 and between 0.5 and 1 with 0.5. Above an eta of 1 the
+// test does not hold.
+constexpr double kFilterEta = 0.5, kFilterEta64 = 1.0;
+double filter_guess(double eta) { return eta <= 0.15 ? 0.8 : (eta <= 0.5 ? 0.5 : 0.3); }
 }  // namespace
 
 // levels with packed kick sources (deeper levels, if they run grid phases at all, gather)
@@ -4487,7 +4498,8 @@ EParams engine_params(hhs_ctx* c, EngineHost* eh, const SoA& P, int n, double dt
     E.tf = eh->tf;
     E.tau_key = eh->tau_key;
     // the bounds are guessed from timesteps that this launch computed
-    E.filter = calc_ts && E.eta <= 1.0 ? 1 : 0;
+    E.tf_guess = filter_guess(E.eta);
+    E.filter = calc_ts && E.eta <= kFilterEta64 ? 1 : 0;
     E.tile_counts = eh->tile_counts;
     E.tile_status = eh->tile_status;
     E.rate_acc = eh->rate_acc;
@@ -4562,6 +4574,7 @@ hhs_status engine_hold_step(hhs_ctx* c, const SoA& P, int n, double dt, bool cal
     EParams E = engine_params(c, eh, P, n, dt, calc_ts, profile, top_level);
     const int pi = prec == HHS_PREC_FP64 ? 0 : 1;
     E.prec_mixed = pi;
+    if (pi == 1 && E.eta > kFilterEta) E.filter = 0;
     const int mid_n = std::min(pi == 0 ? std::min(eh->mid_n, kMidFp64) : eh->mid_n, kMid);
     const cudaError_t e = top_level == 0 && n <= mid_n
                               ? (pi == 0 ? subtree_launch(eh, k_subtree<HHS_PREC_FP64>, E, stream)

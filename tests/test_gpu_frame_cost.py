@@ -180,3 +180,33 @@ def test_step_without_the_filter_where_it_does_not_help(cuda, hhs, kind, n):
     x, y = a.download(), b.download()
     for k in ("x", "y", "z", "vx", "vy", "vz", "ts"):
         assert np.array_equal(x[k], y[k]), k
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("eta", [0.25, 0.5, 1.0])
+def test_step_with_large_timesteps(cuda, hhs, eta, prec):
+    """Rates change with eta from one calculation to the next; a row whose bound was too high is
+    scanned whole in the split phase, which then took 30 to 80% of the step (it takes 4 to 6%)."""
+    p = _phases(hhs, hhs.plummer(9001, 5), 0.125 if eta < 1.0 else 0.25, eta, prec)
+    assert p["split"] < 0.15 * sum(p.values())
+
+
+@pytest.mark.parametrize("n", [1001, 2500])
+def test_rows_whose_bound_was_too_high_fp64(cuda, hhs, oracle, n):
+    """A common velocity of 2^20 leaves FP32 relative velocities of 2^-4: the bounds of the top
+    node, from FP32 rates, exceed many FP64 rates, and the rows are scanned whole."""
+    s = hhs.plummer(n, 5)
+    s["vy"] += 2.0 ** 20
+    ts = oracle.timesteps(s, 0.03)
+    d = hhs.ParticleSystem(n)
+    d.upload(s)
+    ctx = hhs.Context(n, 64, 0.03)
+    hhs.timesteps(ctx, d, n, hhs.PREC_MIXED)  # the same FP32 rates
+    assert np.count_nonzero(0.999 / d.download()["ts"] * ts > 1.0) > n // 20
+    d.upload(s)
+    hhs.hold_step(ctx, d, n, 0.0, 1.0 / 64, True, hhs.PREC_FP64)
+    ctx.check()
+    oracle.hold_step(s, 1.0 / 64, True, 0.03)
+    out = d.download()
+    for k in ("x", "y", "z", "vx", "vy", "vz", "ts"):
+        assert np.array_equal(out[k], s[k]), k
