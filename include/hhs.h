@@ -434,7 +434,9 @@ hhs_status hhs_measure_fma2_peak(double* fp32x2_tflops, void* stream);
  * advances every system by one top-level HOLD step in ONE launch: hardware thread-block
  * clusters take the large systems (largest first, one cluster per system, cluster
  * barriers between phases), then single CTAs take the rest, each split being a
- * per-system (segmented) scan and compaction. Per-system leaf times are kept. */
+ * per-system (segmented) scan and compaction. Per-system leaf times are kept.
+ * FP64 steps equal the sequential order bit for bit; a mixed system's bits follow from the
+ * system and the tuning, not from the other systems of the batch. */
 typedef struct hhs_batch hhs_batch;
 hhs_status hhs_batch_create(int32_t n_sys, const int32_t* offsets, int32_t max_levels,
                             hhs_params params, hhs_batch** out);

@@ -309,6 +309,7 @@ __device__ bool grid_barrier(const EParams& E, Smem& sm, bool stored = true) {
 enum { kModeBlock = 0, kModeGrid = 1, kModeCluster = 2 };
 struct Workers {
     int id, count, mode;
+    int parts;  // clusters: sums are divided as by this many CTAs, whatever their number
 };
 
 // Announces the bulk copies of a tile, by the thread that issues them: of records that an earlier
@@ -388,9 +389,10 @@ __device__ void prof_end(const EParams& E, Smem& sm) {
 // number of source chunks for a node of n sinks
 __device__ __forceinline__ int chunks_for(int n, const Workers& W, bool split_ok, int upc,
                                           int block = kEB) {
-    if (W.mode == kModeBlock || !split_ok) return 1;
+    const int parts = W.mode == kModeCluster ? W.parts : W.count;
+    if (W.mode == kModeBlock || !split_ok || (W.mode == kModeCluster && parts == 1)) return 1;
     const int nsb = (n + block - 1) / block;
-    int c = (upc * W.count + nsb - 1) / nsb;
+    int c = (upc * parts + nsb - 1) / nsb;
     c = c < 1 ? 1 : (c > kMaxChunks ? kMaxChunks : c);
     const int maxc = (n + 63) / 64;  // at least 64 sources per chunk
     return c < maxc ? c : (maxc < 1 ? 1 : maxc);
@@ -2965,6 +2967,59 @@ __device__ __forceinline__ void acc_over(const EParams& E, const MidState& M, co
     for (; q < qn; q += step) one(list[q]);
 }
 
+// The mixed kick of a cluster of cs CTAs with the sums of a cluster of V: the shares that V CTAs
+// would have are dealt to the cs ones whole, or one's groups of 32 sinks to cs / V of them.
+// (Both are powers of two.)
+__device__ __forceinline__ void kick_parts(const EParams& E, MidState& M, int ns, int nk, double dt,
+                                           bool dist, int V, int cs, int rank) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int v0 = 0, v1 = 1, g0 = 0, gs = 1;
+    if (dist && V >= cs) {
+        v0 = rank * (V / cs);
+        v1 = v0 + V / cs;
+    } else if (dist) {
+        gs = cs / V;
+        v0 = rank / gs;
+        v1 = v0 + 1;
+        g0 = rank % gs;
+    }
+    for (int v = v0; v < v1; v++) {
+        const Share sh = share_of(nk, V > 1, V, v);
+        const int ng = (sh.ng - g0 + gs - 1) / gs;  // this CTA's groups of the share
+        for (int it = warp; it < ng * sh.wpg; it += kEB / 32) {
+            const int part = it % sh.wpg, p = sh.s0 + (g0 + it / sh.wpg * gs) * 32 + lane;
+            const bool act = p < sh.s1;
+            const int i = act ? M.kl[p] : 0;
+            float a[3] = {0, 0, 0};
+            if (act) acc_over(E, M, M.kl, part, p < ns ? nk : ns, sh.wpg, i, a);
+            if (sh.wpg > 1) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) M.red.part[it][c][lane] = a[c];
+            } else if (act) {
+                put(&M.vx[i], fma((double)a[0], dt, M.vx[i]), dist, cs);
+                put(&M.vy[i], fma((double)a[1], dt, M.vy[i]), dist, cs);
+                put(&M.vz[i], fma((double)a[2], dt, M.vz[i]), dist, cs);
+            }
+        }
+        if (sh.wpg > 1) {
+            __syncthreads();
+            const int p = sh.s0 + (g0 + warp * gs) * 32 + lane;
+            if (warp < ng && p < sh.s1) {
+                const int i = M.kl[p];
+                double acc[3] = {0, 0, 0};
+                for (int q = 0; q < sh.wpg; q++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+                        acc[c] += (double)M.red.part[warp * sh.wpg + q][c][lane];
+                put(&M.vx[i], fma(acc[0], dt, M.vx[i]), dist, cs);
+                put(&M.vy[i], fma(acc[1], dt, M.vy[i]), dist, cs);
+                put(&M.vz[i], fma(acc[2], dt, M.vz[i]), dist, cs);
+            }
+            if (v + 1 < v1) __syncthreads();  // the next share's partial sums overwrite these
+        }
+    }
+}
+
 }  // namespace mid
 
 // Fine-grained timing inside the cluster subtree solver (profiling only; CTA 0, thread 0):
@@ -3234,9 +3289,10 @@ __device__ void warp_subtree(const EParams& E, MidState& M, const unsigned* memw
 
 // cs, rank: the hardware cluster that runs the subtree (every CTA of it calls mid_hold),
 // or cs = 1 for one CTA alone whatever cluster it belongs to.
-template <int PREC>
+// BATCH: the mixed sums are divided as by a cluster of `parts` CTAs (else parts is not used).
+template <int PREC, bool BATCH = false>
 __device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int n, int level0,
-                                         bool calc0, int dist_n, int cs, int rank) {
+                                         bool calc0, int dist_n, int cs, int rank, int parts = 0) {
     Smem& sm = cta_smem();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -3470,6 +3526,8 @@ __device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int
                         mid::put(&M.vy[i], vy, dist, cs);
                         mid::put(&M.vz[i], vz, dist, cs);
                     }
+                } else if constexpr (BATCH) {
+                    mid::kick_parts(E, M, ns, nk, dt, dist, dist && parts > 1 ? parts : 1, cs, rank);
                 } else {
                     const int items = sh.ng * sh.wpg;
                     for (int it = warp; it < items; it += kEB / 32) {
@@ -3629,7 +3687,8 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     if constexpr (PREC == HHS_PREC_FP64)
                         mid_hold_fp64(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
                     else
-                        mid_hold<PREC>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
+                        mid_hold<PREC, true>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id,
+                                             W.parts);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfCluster, 0.0, sm, lvl);
@@ -4107,11 +4166,17 @@ struct Slot {
     unsigned* rate_acc;
 };
 
+// A mixed system's sums, and so its bits, follow from its own size: the number of CTAs that work on
+// it does not (it follows from the other systems, see batched_shape). Systems of at most parts_n
+// particles are summed as by one CTA.
+constexpr int kBatchParts = 8;
+constexpr int kBatchPartsN = 1024;
 struct BParams {
     EParams E;               // common fields; per-system fields are filled in per system
     const int32_t* offsets;  // [n_sys + 1]
     const int32_t* order;    // systems by decreasing size
     int n_sys, n_big;
+    int parts_n;             // mixed sums of systems above this size are divided in kBatchParts
     unsigned* queues;        // [0] big-system queue, [1] small-system queue, [2 + c] broadcast
     char* cluster_slots;
     char* cta_slots;
@@ -4159,7 +4224,7 @@ __global__ void __launch_bounds__(kEB, 2) k_batched(BParams B) {
         if (idx >= B.n_big) break;
         const int sys = B.order[idx];
         const EParams E = system_params(B, sys, B.cluster_slots + (size_t)cid * B.cluster_slot_bytes);
-        const Workers W{rank, cs, kModeCluster};
+        const Workers W{rank, cs, kModeCluster, E.n_top > B.parts_n ? kBatchParts : 1};
         run_hold<PREC, kModeCluster, false>(E, 0, E.calc_top != 0, W, sm, t);
     }
     // small systems: one CTA per system
@@ -4718,6 +4783,7 @@ struct hhs_batch {
     int big_n = 1024, cluster_size = 8, small_n = 64, units_per_cta = 8, warp_n = 32, packed = 0;
     int mid_n = kMid, mid_dist_n = 96;
     int n_big = 0, n_big64 = 0, n_clusters[2] = {0, 0};  // n_big64: FP64 steps
+    int parts_n = kBatchPartsN;  // big_n, once the caller has set it
     void* arena = nullptr;
     int32_t* d_offsets = nullptr;
     int32_t* d_order = nullptr;
@@ -4879,7 +4945,7 @@ extern "C" hhs_status hhs_batch_set_tuning(hhs_batch* b, int32_t big_n, int32_t 
                                            int32_t units_per_cta) {
     if (!b || big_n < 0 || small_n < 0 || units_per_cta < 1 || units_per_cta > 64)
         return HHS_ERR_INVALID_ARG;
-    b->big_n = big_n;
+    b->big_n = b->parts_n = big_n;
     b->small_n = small_n;
     b->units_per_cta = units_per_cta;
     b->n_big = 0;
@@ -4955,6 +5021,7 @@ extern "C" hhs_status hhs_hold_batched(hhs_batch* b, hhs_particle_system* sys, d
     B.order = b->d_order;
     B.n_sys = b->n_sys;
     B.n_big = pi == 0 ? b->n_big64 : b->n_big;
+    B.parts_n = b->parts_n;
     B.queues = b->d_queues;
     B.cluster_slots = b->cluster_slots;
     B.cta_slots = b->cta_slots;

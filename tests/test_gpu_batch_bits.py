@@ -1,0 +1,34 @@
+"""A mixed system's bits in a batch follow from the system, not from the others of the batch (whose
+sizes decide how many CTAs work on it)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("x", "y", "z", "vx", "vy", "vz", "ts")
+
+
+def _step(hhs, sizes, tuning=None):
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    parts = [hhs.plummer(n, n) for n in sizes]
+    d = hhs.ParticleSystem(int(off[-1]))
+    d.upload({k: np.concatenate([p[k] for p in parts]) for k in parts[0]})
+    b = hhs.Batch(off, 64, 0.03)
+    if tuning:
+        b.set_tuning(**tuning)
+    for _ in range(2):
+        b.step(d, 1.0 / 64, True, hhs.PREC_MIXED)
+    b.check()
+    out = d.download()
+    return {k: out[k][:sizes[0]].copy() for k in KEYS}
+
+
+@pytest.mark.parametrize("n", [641, 800, 1024, 1025, 2049, 3001])
+def test_bits_do_not_depend_on_the_other_systems(cuda, hhs, n):
+    # alone: clusters of 16; 12 more of its size: of 8; 48 more: of 4 (a CTA each for those of at
+    # most 1024 beside a larger one)
+    alone = _step(hhs, [n])
+    for others in ([n] * 12, [n] * 48, [3001], [4001, 100]):
+        other = _step(hhs, [n] + others)
+        for k in KEYS:
+            assert np.array_equal(alone[k], other[k]), (k, len(others))
