@@ -3618,11 +3618,12 @@ __device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int
     mid_mark(E, sm, tm, 61);
 }
 
-// The FP64 solver as a function: the batched kernel has it in three places, and inlined in each
-// it spills (300 systems of up to 640 particles: 9.9 ms, called 9.1).
-__device__ __noinline__ void mid_hold_fp64(const EParams& E, const int32_t* S, int n, int level0,
-                                           bool calc0, int dist_n, int cs, int rank) {
-    mid_hold<HHS_PREC_FP64>(E, S, n, level0, calc0, dist_n, cs, rank);
+// FP64 rows as a function of the batched kernel, which has them in two places: inlined, its other
+// phases spill, and a function that took EParams by reference would put the system's copy of them
+// into local memory (as one for mid_hold did: 400 systems of up to 640 particles 9.3 ms, 8.5 with
+// this; 300 of up to 2048 32.3, 28.8).
+__device__ __noinline__ void ts_rows_fp64(SoA P, const int32_t* S, int n, int i0, int nrow, TsArgs A) {
+    ts_rows<HHS_PREC_FP64>(P, S, n, i0, nrow, A, cta_smem().u.tr);
 }
 
 // True when the kick of level lvl (a grid node with a fast set of at most mid_n) runs its
@@ -3684,11 +3685,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                                        1, W.id - cs, W.count - cs, sm);
                     }
                 } else {
-                    if constexpr (PREC == HHS_PREC_FP64)
-                        mid_hold_fp64(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
-                    else
-                        mid_hold<PREC, true>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id,
-                                             W.parts);
+                    mid_hold<PREC, true>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id, W.parts);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfCluster, 0.0, sm, lvl);
@@ -3774,7 +3771,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     while (T > 8 && (n + T - 1) / T < W.count) T >>= 1;
                     for (int i0 = W.id * T; i0 < n; i0 += W.count * T) {
                         const int nrow = min(T, n - i0);
-                        ts_rows<PREC>(E.P, S, n, i0, nrow, A, sm.u.tr);
+                        ts_rows_fp64(E.P, S, n, i0, nrow, A);
                         if ((int)threadIdx.x < nrow)
                             E.P.ts[list_at(S, i0 + threadIdx.x)] =
                                 ts_of_key<PREC>(sm.u.tr.best[threadIdx.x]);
@@ -4206,7 +4203,7 @@ __device__ __forceinline__ EParams system_params(const BParams& B, int sys, cons
 }
 
 template <int PREC>
-__global__ void __launch_bounds__(kEB, 2) k_batched(BParams B) {
+__global__ void __launch_bounds__(kEB, 2) k_batched(const __grid_constant__ BParams B) {
     Smem& sm = cta_smem();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
