@@ -4827,21 +4827,43 @@ cudaError_t batched_occupancy(int cs, int* clusters) {
 // barriers span fewer CTAs and more systems run side by side). Measured, ms per launch with
 // clusters of 4 / 8 / 16: 32 systems of 64 to 4096 particles (e = 3.3) 16.2 / 11.1 / 6.8, 100
 // (10) 21.6 / 11.6 / 11.8, 200 (21) 23.6 / 13.5 / 18.9, 512 (53) 26.0 / 32.3 / 47.2; 300 of 64 to
-// 2048 (37) 10.4 / 9.8 / 12.8. Where no system exceeds 1024 particles, those above 640 (the largest
-// that one CTA holds in shared memory) get the clusters: 500 systems of 64 to 1024 (51) 3.6 ms
-// with clusters of 4 against 4.6 with every system on a CTA of its own.
+// 2048 (37) 10.4 / 9.8 / 12.8.
+// Where no system exceeds 1024 particles, those above 640 (the largest that one CTA holds in shared
+// memory) get clusters as large as lets all of them start at once: the systems behind them, some
+// of which take several times the others' time, are not to wait for a second round. Mixed ms per
+// launch, clusters / a CTA each: 20 systems of 641 to 1024 2.1 / 3.3, with 400 smaller ones 2.5 / 3.1,
+// 60 2.5 / 4.2 and 4.0 / 4.4; where they are more than there are clusters of 4, 100 3.1 / 4.8 and with
+// 400 smaller ones 4.2 / 4.3, 170 4.7 / 4.7 and 5.7 / 4.8. So above that number only batches of at
+// most twice as many systems in all get them.
+bool batched_clusters(int cs, int* c0, int* c1) {
+    if (batched_occupancy<HHS_PREC_FP64>(cs, c0) == cudaSuccess &&
+        batched_occupancy<HHS_PREC_MIXED>(cs, c1) == cudaSuccess && *c0 > 0 && *c1 > 0)
+        return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
 bool batched_shape(hhs_batch* b, int* c0, int* c1) {
     b->big_n = b->n_max_sys > 1024 ? 1024 : kMid;
+    int large = 0, want = 4;
     double e = 0.0;
     for (const int n : b->sizes)
-        if (n > b->big_n) e += std::pow((double)n / b->n_max_sys, 2.33);
-    // the portable size is the fallback
-    for (const int cs : {e < 8.0 ? 16 : (e < 40.0 ? 8 : 4), 8}) {
+        if (n > b->big_n) {
+            e += std::pow((double)n / b->n_max_sys, 2.33);
+            large++;
+        }
+    if (b->n_max_sys > 1024) {
+        want = e < 8.0 ? 16 : (e < 40.0 ? 8 : 4);
+    } else {
+        for (const int cs : {4, 8, 16}) {
+            if (!batched_clusters(cs, c0, c1)) continue;
+            if (large <= *c1) want = cs;
+            if (cs == 4 && large > *c1 && b->n_sys > 2 * *c1) b->big_n = 1024;
+        }
+    }
+    for (const int cs : {want, 8}) {  // the portable size is the fallback
         b->cluster_size = cs;
-        if (batched_occupancy<HHS_PREC_FP64>(cs, c0) == cudaSuccess &&
-            batched_occupancy<HHS_PREC_MIXED>(cs, c1) == cudaSuccess && *c0 > 0 && *c1 > 0)
-            return true;
-        (void)cudaGetLastError();
+        if (batched_clusters(cs, c0, c1)) return true;
     }
     return false;
 }

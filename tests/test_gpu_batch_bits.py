@@ -32,3 +32,33 @@ def test_bits_do_not_depend_on_the_other_systems(cuda, hhs, n):
         other = _step(hhs, [n] + others)
         for k in KEYS:
             assert np.array_equal(alone[k], other[k]), (k, len(others))
+
+
+def test_many_small_systems_take_no_longer_than_a_cta_each(cuda, hhs):
+    """Default tuning against every system on a CTA of its own, where more systems exceed 640
+    particles than there are clusters and many smaller ones wait behind them."""
+    r = np.random.default_rng(3)
+    sizes = np.exp(r.uniform(np.log(64), np.log(1024), 500)).astype(int)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    parts = [hhs.plummer(int(n), int(n)) for n in sizes]
+    s = {k: np.concatenate([p[k] for p in parts]) for k in parts[0]}
+    d = hhs.ParticleSystem(int(off[-1]))
+    b = hhs.Batch(off, 64, 0.03)
+
+    def ms():
+        best = 1e30
+        for _ in range(5):
+            d.upload(s)
+            e0, e1 = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+            cuda.cuda.synchronize()
+            e0.record()
+            b.step(d, 1.0 / 64, True, hhs.PREC_MIXED)
+            e1.record()
+            cuda.cuda.synchronize()
+            b.check()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    default = ms()
+    b.set_tuning(big_n=1024)
+    assert default < 1.15 * ms()
