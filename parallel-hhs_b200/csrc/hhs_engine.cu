@@ -4157,7 +4157,6 @@ struct Slot {
     int32_t* fast_lists;
     int32_t* slow_lists;
     hhs_partition* counts;
-    double* ts_part;
     double* k_part;
     int* tile_counts;
     unsigned* rate_acc;
@@ -4178,7 +4177,7 @@ struct BParams {
     char* cluster_slots;
     char* cta_slots;
     size_t cluster_slot_bytes, cta_slot_bytes;
-    size_t off_lists, off_counts, off_ts, off_k, off_tiles, off_rate;
+    size_t off_lists, off_counts, off_k, off_tiles, off_rate;
     double* leaf_times;      // [n_sys]
 };
 
@@ -4194,7 +4193,6 @@ __device__ __forceinline__ EParams system_params(const BParams& B, int sys, cons
     E.fast_lists = reinterpret_cast<int32_t*>(p + B.off_lists);
     E.slow_lists = E.fast_lists + lists;
     E.counts = reinterpret_cast<hhs_partition*>(p + B.off_counts);
-    E.ts_part = reinterpret_cast<double*>(p + B.off_ts);
     E.k_part = reinterpret_cast<double*>(p + B.off_k);
     E.tile_counts = reinterpret_cast<int*>(p + B.off_tiles);
     E.rate_acc = reinterpret_cast<unsigned*>(p + B.off_rate);
@@ -4791,7 +4789,7 @@ struct hhs_batch {
     char* cluster_slots = nullptr;
     char* cta_slots = nullptr;
     size_t cluster_slot_bytes = 0, cta_slot_bytes = 0;
-    size_t off_lists = 0, off_counts = 0, off_ts = 0, off_k = 0, off_tiles = 0, off_rate = 0;
+    size_t off_lists = 0, off_counts = 0, off_k = 0, off_tiles = 0, off_rate = 0;
     int max_clusters = 0, max_ctas = 0;
     std::vector<int> sizes, order;
 };
@@ -4872,10 +4870,9 @@ size_t slot_layout(int n, int levels, int chunks, size_t* off) {
     size_t p = 0;
     off[0] = p; p += al(sizeof(int32_t) * 2 * (size_t)levels * n);          // lists
     off[1] = p; p += al(sizeof(hhs_partition) * (size_t)levels);            // counts
-    off[2] = p; p += al(sizeof(double) * (size_t)chunks * n);               // ts partials
-    off[3] = p; p += al(sizeof(double) * (size_t)(chunks * 3 > 6 ? chunks * 3 : 6) * n);
-    off[4] = p; p += al(sizeof(int) * (size_t)(n / kEB + 2));               // tile counts
-    off[5] = p; p += al(sizeof(unsigned) * (size_t)n);                      // rate_acc
+    off[2] = p; p += al(sizeof(double) * (size_t)(chunks * 3 > 6 ? chunks * 3 : 6) * n);
+    off[3] = p; p += al(sizeof(int) * (size_t)(n / kEB + 2));               // tile counts
+    off[4] = p; p += al(sizeof(unsigned) * (size_t)n);                      // rate_acc
     return p;
 }
 }  // namespace
@@ -4912,14 +4909,14 @@ extern "C" hhs_status hhs_batch_create(int32_t n_sys, const int32_t* offsets, in
     b->n_clusters[1] = c1;
     b->max_clusters = c0 > c1 ? c0 : c1;
     b->max_ctas = b->max_clusters * b->cluster_size;
-    size_t offc[6], offs[6];
+    size_t offc[5], offs[5];
     b->cluster_slot_bytes = slot_layout(b->n_max_sys, b->max_levels, kMaxChunks, offc);
     b->cta_slot_bytes = slot_layout(b->n_max_sys, b->max_levels, 1, offs);
     // both slot kinds use the same offsets up to their own sizes: lists and counts first
     b->off_lists = offc[0]; b->off_counts = offc[1];
     // offsets beyond counts differ; keep the larger (cluster) layout for both
     b->cta_slot_bytes = b->cluster_slot_bytes;
-    b->off_ts = offc[2]; b->off_k = offc[3]; b->off_tiles = offc[4]; b->off_rate = offc[5];
+    b->off_k = offc[2]; b->off_tiles = offc[3]; b->off_rate = offc[4];
     (void)offs;
     const size_t head = al(sizeof(int32_t) * (n_sys + 1)) + al(sizeof(int32_t) * n_sys) +
                         al(sizeof(unsigned) * (2 + b->max_clusters)) + al(sizeof(double) * n_sys) +
@@ -5046,7 +5043,7 @@ extern "C" hhs_status hhs_hold_batched(hhs_batch* b, hhs_particle_system* sys, d
     B.cta_slots = b->cta_slots;
     B.cluster_slot_bytes = b->cluster_slot_bytes;
     B.cta_slot_bytes = b->cta_slot_bytes;
-    B.off_lists = b->off_lists; B.off_counts = b->off_counts; B.off_ts = b->off_ts;
+    B.off_lists = b->off_lists; B.off_counts = b->off_counts;
     B.off_k = b->off_k; B.off_tiles = b->off_tiles; B.off_rate = b->off_rate;
     B.leaf_times = b->d_leaf;
     cudaLaunchConfig_t cfg = {};

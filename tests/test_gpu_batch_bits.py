@@ -62,3 +62,18 @@ def test_many_small_systems_take_no_longer_than_a_cta_each(cuda, hhs):
     default = ms()
     b.set_tuning(big_n=1024)
     assert default < 1.15 * ms()
+
+
+def test_scratch_of_a_batch(cuda, hhs):
+    """A slot holds the kick's partial sums (32 chunks of three components) and the level lists, and
+    every CTA and cluster of the launch has one: no partial timesteps (a quarter more)."""
+    n, slots = 4096, 148 * 2 + 148 * 2 // 4
+    b = hhs.Batch(np.array([0, 64], dtype=np.int32), 1, 0.03)  # loads the kernel
+    cuda.cuda.synchronize()
+    free = cuda.cuda.mem_get_info()[0]
+    c = hhs.Batch(np.array([0, n], dtype=np.int32), 1, 0.03)
+    used = free - cuda.cuda.mem_get_info()[0]
+    per_slot = n * (32 * 3 * 8 + 2 * 4 + 4) + 4096
+    assert used <= slots * per_slot + (4 << 20)
+    c.destroy()
+    b.destroy()
