@@ -441,8 +441,10 @@ typedef struct hhs_batch hhs_batch;
 hhs_status hhs_batch_create(int32_t n_sys, const int32_t* offsets, int32_t max_levels,
                             hhs_params params, hhs_batch** out);
 hhs_status hhs_batch_destroy(hhs_batch* b);
-/* big_n: systems with more particles run on a thread-block cluster; small_n: inside a
- * system, nodes with at most small_n particles run on one CTA; units_per_cta as above. */
+/* big_n: systems with more particles run on a thread-block cluster, in either precision
+ * (default: 640 in FP64; in mixed precision 1024, or 640 for some batches without a larger
+ * system; the clusters have 4, 8 or 16 CTAs, by the sizes); small_n: inside a system, nodes
+ * with at most small_n particles run on one CTA; units_per_cta as above. */
 hhs_status hhs_batch_set_tuning(hhs_batch* b, int32_t big_n, int32_t small_n,
                                 int32_t units_per_cta);
 /* Subtrees of at most mid_n (<= 640) particles run from shared memory: on the system's
@@ -455,8 +457,9 @@ typedef struct {
     double ms_per_step;      /* filled by hhs_batch_autotune */
 } hhs_batch_tuning;
 /* Batched autotuner: times hhs_hold_batched on the caller's systems for a grid of
- * (big_n, units_per_cta, mid_dist_n) candidates -- the state, per-system leaf times and
- * work counters restored before every trial and at the end -- and keeps the fastest.
+ * (big_n, units_per_cta, mid_dist_n) candidates, the current big_n among them -- the state,
+ * per-system leaf times and work counters restored before every trial and at the end -- and
+ * keeps the fastest, its big_n for steps of `prec` only.
  * out (optional) receives it; table (optional, capacity entries) every candidate timed,
  * *count (optional) their number. Allocates a snapshot of the state: call it outside
  * any timed or captured region. */

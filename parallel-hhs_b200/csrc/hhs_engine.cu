@@ -4775,10 +4775,11 @@ hhs_status engine_shard_kick(hhs_ctx* c, const SoA& P, const int32_t* F, const i
 struct hhs_batch {
     int n_sys = 0, n_total = 0, n_max_sys = 0, max_levels = 0;
     hhs_params params{0.03, 0.0};
-    int big_n = 1024, cluster_size = 8, small_n = 64, units_per_cta = 8, warp_n = 32, packed = 0;
+    int big_n[2] = {kMid, 1024};  // FP64, mixed: larger systems (n_big of them) get a cluster
+    int n_big[2] = {0, 0}, n_clusters[2] = {0, 0};
+    int cluster_size = 8, small_n = 64, units_per_cta = 8, warp_n = 32, packed = 0;
     int mid_n = kMid, mid_dist_n = 96;
-    int n_big = 0, n_big64 = 0, n_clusters[2] = {0, 0};  // n_big64: FP64 steps
-    int parts_n = kBatchPartsN;  // big_n, once the caller has set it
+    int parts_n = kBatchPartsN;  // big_n of mixed steps, once the caller or the tuner has set it
     void* arena = nullptr;
     int32_t* d_offsets = nullptr;
     int32_t* d_order = nullptr;
@@ -4842,11 +4843,14 @@ bool batched_clusters(int cs, int* c0, int* c1) {
 }
 
 bool batched_shape(hhs_batch* b, int* c0, int* c1) {
-    b->big_n = b->n_max_sys > 1024 ? 1024 : kMid;
+    // FP64 systems that one CTA does not hold in shared memory get a cluster (400 systems of 64 to
+    // 2048: 34.5 ms, with 1024 as in mixed 41.5)
+    int& big_n = b->big_n[1];
+    big_n = b->n_max_sys > 1024 ? 1024 : kMid;
     int large = 0, want = 4;
     double e = 0.0;
     for (const int n : b->sizes)
-        if (n > b->big_n) {
+        if (n > big_n) {
             e += std::pow((double)n / b->n_max_sys, 2.33);
             large++;
         }
@@ -4856,7 +4860,7 @@ bool batched_shape(hhs_batch* b, int* c0, int* c1) {
         for (const int cs : {4, 8, 16}) {
             if (!batched_clusters(cs, c0, c1)) continue;
             if (large <= *c1) want = cs;
-            if (cs == 4 && large > *c1 && b->n_sys > 2 * *c1) b->big_n = 1024;
+            if (cs == 4 && large > *c1 && b->n_sys > 2 * *c1) big_n = 1024;
         }
     }
     for (const int cs : {want, 8}) {  // the portable size is the fallback
@@ -4864,6 +4868,12 @@ bool batched_shape(hhs_batch* b, int* c0, int* c1) {
         if (batched_clusters(cs, c0, c1)) return true;
     }
     return false;
+}
+
+void batch_set_big(hhs_batch* b, int pi, int big_n) {
+    b->big_n[pi] = big_n;
+    b->n_big[pi] = 0;
+    for (const int n : b->sizes) b->n_big[pi] += n > big_n ? 1 : 0;
 }
 
 size_t slot_layout(int n, int levels, int chunks, size_t* off) {
@@ -4940,12 +4950,7 @@ extern "C" hhs_status hhs_batch_create(int32_t n_sys, const int32_t* offsets, in
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_order, b->order.data(), sizeof(int32_t) * n_sys, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { cudaFree(b->arena); delete b; return hhs_from_cuda(e); }
-    // FP64 systems that one CTA does not hold in shared memory get a cluster unless the caller's
-    // tuning says otherwise (400 systems of 64 to 2048: 34.5 ms, with 1024 as in mixed 41.5)
-    for (int k = 0; k < n_sys; k++) {
-        if (b->sizes[b->order[k]] > b->big_n) b->n_big = k + 1;
-        if (b->sizes[b->order[k]] > kMid) b->n_big64 = k + 1;
-    }
+    for (int pi = 0; pi < 2; pi++) batch_set_big(b, pi, b->big_n[pi]);
     *out = b;
     return HHS_OK;
 }
@@ -4961,13 +4966,10 @@ extern "C" hhs_status hhs_batch_set_tuning(hhs_batch* b, int32_t big_n, int32_t 
                                            int32_t units_per_cta) {
     if (!b || big_n < 0 || small_n < 0 || units_per_cta < 1 || units_per_cta > 64)
         return HHS_ERR_INVALID_ARG;
-    b->big_n = b->parts_n = big_n;
+    for (int pi = 0; pi < 2; pi++) batch_set_big(b, pi, big_n);
+    b->parts_n = big_n;
     b->small_n = small_n;
     b->units_per_cta = units_per_cta;
-    b->n_big = 0;
-    for (int k = 0; k < b->n_sys; k++)
-        if (b->sizes[b->order[k]] > b->big_n) b->n_big = k + 1;
-    b->n_big64 = b->n_big;
     return HHS_OK;
 }
 
@@ -5036,7 +5038,7 @@ extern "C" hhs_status hhs_hold_batched(hhs_batch* b, hhs_particle_system* sys, d
     B.offsets = b->d_offsets;
     B.order = b->d_order;
     B.n_sys = b->n_sys;
-    B.n_big = pi == 0 ? b->n_big64 : b->n_big;
+    B.n_big = b->n_big[pi];
     B.parts_n = b->parts_n;
     B.queues = b->d_queues;
     B.cluster_slots = b->cluster_slots;
@@ -5098,14 +5100,24 @@ extern "C" hhs_status hhs_batch_autotune(hhs_batch* b, hhs_particle_system* sys,
     };
     hhs_stats stats_saved{};
     cudaMemcpyAsync(&stats_saved, b->d_stats, sizeof(hhs_stats), cudaMemcpyDeviceToHost, s);
-    const hhs_batch_tuning cur{b->big_n, b->small_n, b->units_per_cta, b->mid_n, b->mid_dist_n, 0.0};
+    const int pi = prec == HHS_PREC_FP64 ? 0 : 1, parts_n = b->parts_n;
+    const hhs_batch_tuning cur{b->big_n[pi], b->small_n, b->units_per_cta, b->mid_n, b->mid_dist_n, 0.0};
+    // big_n is the timed precision's alone
+    auto apply = [&](const hhs_batch_tuning& t) {
+        batch_set_big(b, pi, t.big_n);
+        if (pi == 1) b->parts_n = t.big_n == cur.big_n ? parts_n : t.big_n;
+        b->units_per_cta = t.units_per_cta;
+        b->mid_dist_n = t.mid_dist_n;
+    };
     hhs_batch_tuning best = cur;
     best.ms_per_step = 1e300;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     st = copy_all(true);
-    const int big_c[] = {512, 1024, 2048};
+    // the current big_n is one of the candidates
+    const bool listed = cur.big_n == 1024 || cur.big_n == 2048;
+    const int big_c[] = {listed ? 512 : cur.big_n, 1024, 2048};
     const int upc_c[] = {8, 16};
     const int dist_c[] = {64, 96};
     constexpr int kTimed = 3;
@@ -5115,8 +5127,7 @@ extern "C" hhs_status hhs_batch_autotune(hhs_batch* b, hhs_particle_system* sys,
             for (int dn : dist_c) {
                 if (st != HHS_OK) break;
                 hhs_batch_tuning t{big, cur.small_n, upc, cur.mid_n, dn, 0.0};
-                if ((st = hhs_batch_set_tuning(b, t.big_n, t.small_n, t.units_per_cta)) != HHS_OK) break;
-                if ((st = hhs_batch_set_mid(b, t.mid_n, t.mid_dist_n)) != HHS_OK) break;
+                apply(t);
                 st = copy_all(false);
                 if (st == HHS_OK) st = hhs_hold_batched(b, sys, dt, 1, prec, stream);
                 if (st == HHS_OK) st = copy_all(false);
@@ -5142,9 +5153,7 @@ extern "C" hhs_status hhs_batch_autotune(hhs_batch* b, hhs_particle_system* sys,
     cudaFree(leaf);
     hhs_particle_system_free(&snap);
     if (count) *count = k;
-    const hhs_batch_tuning pick = (st == HHS_OK && st2 == HHS_OK) ? best : cur;
-    hhs_batch_set_tuning(b, pick.big_n, pick.small_n, pick.units_per_cta);
-    hhs_batch_set_mid(b, pick.mid_n, pick.mid_dist_n);
+    apply(st == HHS_OK && st2 == HHS_OK ? best : cur);
     if (st == HHS_OK) st = st2;
     if (st == HHS_OK && out) *out = best;
     return st;

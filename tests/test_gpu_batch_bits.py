@@ -77,3 +77,19 @@ def test_scratch_of_a_batch(cuda, hhs):
     assert used <= slots * per_slot + (4 << 20)
     c.destroy()
     b.destroy()
+
+
+def test_autotune_keeps_to_its_precision(cuda, hhs):
+    """The tuner times the batch's own big_n among its candidates, the default too, and sets that of
+    the precision it times only."""
+    sizes = [700, 900, 64, 300]
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    parts = [hhs.plummer(n, n) for n in sizes]
+    d = hhs.ParticleSystem(int(off[-1]))
+    d.upload({k: np.concatenate([p[k] for p in parts]) for k in parts[0]})
+    b = hhs.Batch(off, 64, 0.03)
+    for prec in (hhs.PREC_FP64, hhs.PREC_MIXED):
+        assert 640 in {t["big_n"] for t in b.autotune(d, 1.0 / 64, prec)[1]}
+    b.set_tuning(big_n=800)
+    b.autotune(d, 1.0 / 64, hhs.PREC_MIXED)
+    assert 800 in {t["big_n"] for t in b.autotune(d, 1.0 / 64, hhs.PREC_FP64)[1]}
