@@ -5,6 +5,9 @@
 // src/kick.cuh:59-155), but on SoA FP64 arrays addressed through index lists, with
 // the tail tile loaded correctly (the reference returns before the cooperative load,
 // src/timestep.cuh:70) and every launch sized from device-resident counts.
+#include <algorithm>
+#include <cmath>
+
 #include "hhs_common.cuh"
 #include "hhs_kernels.h"
 #include "hhs_kick64.cuh"
@@ -16,6 +19,7 @@ using namespace hhs;
 namespace {
 
 constexpr int kKickBlock = 128;
+constexpr int kSms = 148;  // of a B200
 
 __device__ __forceinline__ int list_at(const int32_t* list, int i) { return ts_list_at(list, i); }
 
@@ -185,7 +189,7 @@ __global__ void __launch_bounds__(kKickBlock)
 
 // ---------------------------------------------------------------- standalone kicks
 // kick_slow / kick_sf of the reference API: sinks sink[0..n), sources src[0..m).
-// FP64: a CTA per block of 8 sinks, terms evaluated by seven of its warps and added in source
+// FP64, unless the sources are few: a CTA per block of 8 sinks, terms evaluated by seven of its warps and added in source
 // order by the eighth (hhs_kick64.cuh).
 __global__ void __launch_bounds__(kK64Threads, 2)
     k_kick_pair_fp64(SoA K, double* __restrict__ ax_out, double* __restrict__ ay_out,
@@ -302,6 +306,83 @@ __global__ void __launch_bounds__(32 * kPmWarps, 3)
     }
 }
 
+// Many sinks and few sources (few_sources): a thread per sink, which adds its terms one after another.
+// FP64: the order, and so the bits, of the form above.
+__global__ void __launch_bounds__(kKickBlock)
+    k_kick_few_fp64(SoA K, double* __restrict__ ax_out, double* __restrict__ ay_out,
+                    double* __restrict__ az_out, SoA S, int n, int m, double dtfac) {
+    __shared__ double sx[kKickBlock], sy[kKickBlock], sz[kKickBlock], sm[kKickBlock];
+    const int i = blockIdx.x * kKickBlock + threadIdx.x;
+    const bool active = i < n;
+    const double xi = active ? K.x[i] : 0.0, yi = active ? K.y[i] : 0.0,
+                 zi = active ? K.z[i] : 0.0;
+    double ax = 0, ay = 0, az = 0;
+    for (int jt = 0; jt < m; jt += kKickBlock) {
+        const int j = jt + threadIdx.x;
+        if (j < m) {
+            sx[threadIdx.x] = S.x[j]; sy[threadIdx.x] = S.y[j]; sz[threadIdx.x] = S.z[j];
+            sm[threadIdx.x] = S.m[j];
+        }
+        __syncthreads();
+        if (active) {
+            const int jn = min(kKickBlock, m - jt);
+            for (int jl = 0; jl < jn; jl++)
+                kick_pair_fp64(f64_sub(sx[jl], xi), f64_sub(sy[jl], yi), f64_sub(sz[jl], zi), sm[jl],
+                               ax, ay, az);
+        }
+        __syncthreads();
+    }
+    if (!active) return;
+    if (ax_out) { ax_out[i] = ax; ay_out[i] = ay; az_out[i] = az; }
+    K.vx[i] = f64_add(K.vx[i], f64_mul(ax, dtfac));
+    K.vy[i] = f64_add(K.vy[i], f64_mul(ay, dtfac));
+    K.vz[i] = f64_add(K.vz[i], f64_mul(az, dtfac));
+}
+
+__global__ void __launch_bounds__(kKickBlock)
+    k_kick_few_mixed(SoA K, double* __restrict__ ax_out, double* __restrict__ ay_out,
+                     double* __restrict__ az_out, SoA S, int n, int m, double dtfac) {
+    __shared__ float4 sA[kKickBlock], sB[kKickBlock];
+    const int i = blockIdx.x * kKickBlock + threadIdx.x;
+    const bool active = i < n;
+    DS xi{0, 0}, yi{0, 0}, zi{0, 0};
+    if (active) { xi = ds_split(K.x[i]); yi = ds_split(K.y[i]); zi = ds_split(K.z[i]); }
+    float acc[3] = {0, 0, 0}, cmp[3] = {0, 0, 0};
+    for (int jt = 0; jt < m; jt += kKickBlock) {
+        const int j = jt + threadIdx.x;
+        if (j < m) {
+            const DS a = ds_split(S.x[j]), b = ds_split(S.y[j]), c = ds_split(S.z[j]);
+            sA[threadIdx.x] = make_float4(a.hi, b.hi, c.hi, (float)S.m[j]);
+            sB[threadIdx.x] = make_float4(a.lo, b.lo, c.lo, 0.0f);
+        }
+        __syncthreads();
+        if (active) {
+            const int jn = min(kKickBlock, m - jt);
+            for (int jl = 0; jl < jn; jl++) {
+                const float4 A = sA[jl], B = sB[jl];
+                const float dx = ds_diff(A.x, B.x, xi.hi, xi.lo);
+                const float dy = ds_diff(A.y, B.y, yi.hi, yi.lo);
+                const float dz = ds_diff(A.z, B.z, zi.hi, zi.lo);
+                const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                if (d2 == 0.0f) continue;
+                const float ri = rsqrt_nr(d2);
+                const float mr3 = A.w * ri * ri * ri;
+                kahan_add(acc[0], cmp[0], dx * mr3);
+                kahan_add(acc[1], cmp[1], dy * mr3);
+                kahan_add(acc[2], cmp[2], dz * mr3);
+            }
+        }
+        __syncthreads();
+    }
+    if (!active) return;
+    const double a0 = (double)acc[0] - cmp[0], a1 = (double)acc[1] - cmp[1],
+                 a2 = (double)acc[2] - cmp[2];
+    if (ax_out) { ax_out[i] = a0; ay_out[i] = a1; az_out[i] = a2; }
+    K.vx[i] += a0 * dtfac;
+    K.vy[i] += a1 * dtfac;
+    K.vz[i] += a2 * dtfac;
+}
+
 // ---------------------------------------------------------------- drift / gathers
 // pos += vel*h (src/drift.cuh:24-26) over the slow list of a split level.
 __global__ void k_drift_slow(SoA P, const int32_t* __restrict__ L,
@@ -358,7 +439,7 @@ __global__ void k_gather_split(SoA T, SoA Ls, int32_t* __restrict__ lpar, SoA Fs
 inline int grid_for(int n, int block) { return (n + block - 1) / block; }
 inline int grid_stride(int n, int block) {
     int g = grid_for(n, block);
-    return g < 148 * 8 ? (g > 0 ? g : 1) : 148 * 8;
+    return g < kSms * 8 ? (g > 0 ? g : 1) : kSms * 8;
 }
 
 }  // namespace
@@ -374,7 +455,7 @@ hhs_status launch_timesteps(const SoA& P, const int32_t* list, int n, double eta
     const TsArgs A{eta, eta_s2, (float)(1.0 / eta_s2), (float)(1.0 / eta)};
     // rows of a CTA: the rows share the columns' conversion, but every SM should have its four
     // CTAs (16384 particles: 261 us with 32 rows, 363 with 64; 32768: 823 with 32, 992 with 64)
-    const int rows = hi - po.lo, T = rows <= 32 * 148 ? 8 : (rows <= 64 * 148 ? 16 : kTsMaxRows);
+    const int rows = hi - po.lo, T = rows <= 32 * kSms ? 8 : (rows <= 64 * kSms ? 16 : kTsMaxRows);
     if (prec == HHS_PREC_FP64)
         k_timesteps<HHS_PREC_FP64><<<grid_for(rows, T), kTsThreads, 0, stream>>>(P, list, n, T, A, po);
     else
@@ -404,11 +485,32 @@ hhs_status launch_kick_level(const SoA& P, const int32_t* fast_list,
     return HHS_OK;
 }
 
+// Whether a thread per sink is the faster form for n sinks and m sources. Its time is m source
+// visits one after another; the other forms take whole rounds of CTAs for 8 (FP64) or 32 sinks each,
+// which few sources leave mostly idle. The models below are fits of the measured microseconds
+// (thread / CTA), FP64: 4096 x 10 6.2 / 8.3, x 64 14.4 / 8.3, 32768 x 10 6.2 / 43, x 300 55 / 74, x 1500
+// 258 / 207, 100000 x 100 36 / 140, x 300 99 / 213; mixed: 32768 x 10 6.2 / 8.3, x 64 10.3 / 10.3,
+// x 224 24.6 / 14.8, 100000 x 20 8.3 / 18.5, x 100 23 / 25, x 300 62 / 49.
+static bool few_sources(int n, int m, hhs_precision prec) {
+    const double dn = n, dm = m;
+    if (prec == HHS_PREC_FP64) {
+        const double rounds = std::ceil(dn / (kK64Sinks * 2 * kSms)), stages = (m + kK64Sources - 1) / kK64Sources;
+        return 2.5 + 0.17 * dm * std::max(1.0, dn / 55000.0) < rounds * (1.0 + 1.9 * stages);
+    }
+    return 3.6 + 0.0915 * dm * std::max(1.0, dn / 48000.0) < 1.4 + 1.26e-4 * dn + 1.3e-6 * dn * dm;
+}
+
 hhs_status launch_kick_pair(const SoA& sink, double* ax, double* ay, double* az,
                             const SoA& src, int n_sink, int n_src, double dtfac,
                             hhs_precision prec, cudaStream_t stream) {
     if (n_sink <= 0) return HHS_OK;
-    if (prec == HHS_PREC_FP64) {
+    if (few_sources(n_sink, n_src, prec)) {
+        const int grid = grid_for(n_sink, kKickBlock);
+        if (prec == HHS_PREC_FP64)
+            k_kick_few_fp64<<<grid, kKickBlock, 0, stream>>>(sink, ax, ay, az, src, n_sink, n_src, dtfac);
+        else
+            k_kick_few_mixed<<<grid, kKickBlock, 0, stream>>>(sink, ax, ay, az, src, n_sink, n_src, dtfac);
+    } else if (prec == HHS_PREC_FP64) {
         constexpr int bytes = (int)sizeof(Kick64Smem);
         HHS_CUDA_TRY(cudaFuncSetAttribute(k_kick_pair_fp64,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
