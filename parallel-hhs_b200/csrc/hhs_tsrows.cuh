@@ -38,6 +38,10 @@ __device__ __forceinline__ int ts_list_at(const int32_t* list, int i) { return l
 constexpr int kTsThreads = 256;
 constexpr int kTsCols = 2 * kTsThreads;  // columns of a tile
 constexpr int kTsSeed = 32;              // columns that every row evaluates first
+// No more columns than these are evaluated without a test, whose phases cost a small call more than
+// its pairs: FP64 / mixed 7 particles 8.3 / 8.3 -> 5.2 / 4.2 us, 33 8.3 / 8.3 -> 6.2 / 4.4 (a thread a
+// particle: 8.3 / 4.2, 24.6 / 6.2). At 64 the evaluation is still the shorter (6.2 / 5.0 against 9.3 / 8.3).
+constexpr int kTsDirect = 64;
 constexpr int kTsCap = 2048;             // pairs listed at a time
 constexpr unsigned kTsBatch = 64;        // listed pairs that are worth evaluating together
 constexpr int kTsMaxRows = 32;
@@ -219,14 +223,19 @@ __device__ __forceinline__ void ts_rows(const SoA& P, const int32_t* list, int n
     }
     if (tid < kTsMaxRows) sm.best[tid] = 0ull;
     if (tid == 0) sm.cnt = 0u;
-    const double sample = tid < 6 * 32 ? ts_centre_sample(P, list, n, tid >> 5) : 0.0;
+    const int seed = n <= kTsDirect ? kTsDirect : kTsSeed;
+    const double sample = n > kTsDirect && tid < 6 * 32 ? ts_centre_sample(P, list, n, tid >> 5) : 0.0;
     __syncthreads();
-    for (int k = tid; k < nrow * kTsSeed; k += kTsThreads) {
-        const int r = k / kTsSeed, j = k % kTsSeed;
+    for (int k = tid; k < nrow * seed; k += kTsThreads) {
+        const int r = k / seed, j = k % seed;
         if (j < n && j != i0 + r) {
             const unsigned long long q = ts_key<PREC>(sm.row[r], ts_load(P, ts_list_at(list, j)), A);
             if (q > sm.best[r]) atomicMax(&sm.best[r], q);
         }
+    }
+    if (n <= kTsDirect) {
+        __syncthreads();
+        return;
     }
     __syncwarp();
     const double median = ts_median(sample);

@@ -59,3 +59,38 @@ def test_kick_sf_mixed_tile_edges(cuda, hhs, oracle, n_sink, n_src):
     mag = np.where(r2 > 0, src["m"][None, :] / np.where(r2 > 0, r2, 1.0), 0.0).sum(1)
     acc = oracle.kick(sink, src, 1.0)
     assert np.all(np.abs(dv - acc) <= 5e-7 * mag + 1e-15)
+
+
+@pytest.mark.parametrize("n", [2, 7, 8, 31, 32, 63, 64, 65])
+@pytest.mark.parametrize("eta", [0.03, 1.5])
+def test_timesteps_of_few_particles(cuda, hhs, oracle, n, eta):
+    """Up to 64 particles every pair is evaluated without a test."""
+    s = hhs.plummer(n, 3)
+    ctx = hhs.Context(n, 8, eta)
+    d = _upload(hhs, s)
+    ref = oracle.timesteps(s, eta)
+    hhs.timesteps(ctx, d, n, hhs.PREC_FP64)
+    assert np.array_equal(d.download()["ts"], ref)
+    hhs.timesteps(ctx, d, n, hhs.PREC_MIXED)
+    assert np.all(np.abs(d.download()["ts"] - ref) <= 2e-6 * ref)
+
+
+def test_timesteps_of_few_particles_take_less_than_of_many(cuda, hhs):
+    """Mixed: 16 particles against 256, whose rows go through the test's phases (as those of 16 did)."""
+    def us(n):
+        d = _upload(hhs, hhs.plummer(n, 3))
+        ctx = hhs.Context(n, 8, 0.03)
+        best = 1e30
+        for _ in range(10):
+            e0, e1 = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+            cuda.cuda.synchronize()
+            cuda.cuda._sleep(400000)
+            e0.record()
+            for _ in range(50):
+                hhs.timesteps(ctx, d, n, hhs.PREC_MIXED)
+            e1.record()
+            cuda.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1) * 20.0)
+        return best
+
+    assert us(16) < 0.75 * us(256)
