@@ -284,7 +284,7 @@ hhs_status hhs_ipc_close(hhs_particle_system* view);
 
 /* Exact exclusive prefix sum of int32 values (the contract of
  * scan_predicate_small/large, src/split.cuh:438-565): one decoupled-lookback pass below
- * 2^18 values, two passes over chunks (chunk sums, then chunk scans) up to 2^25, and from
+ * 2^19 values, two passes over chunks (chunk sums, then chunk scans) up to 2^25, and from
  * 2^25 values (16-byte aligned input and output) one streamed pass: a cooperative launch
  * of resident CTAs that bulk-copy chunks into shared memory and exchange chunk
  * aggregates two rounds ahead (unaligned pointers keep the two-pass form).

@@ -69,14 +69,16 @@ __global__ void __launch_bounds__(kScanBlock, 6)
 // two steps over contiguous chunks of whole tiles, one chunk per CTA: sum the chunk,
 // then scan it from the sum of the chunks before it.
 //  - Two-kernel form: a chunk-sum kernel and a chunk-scan kernel over the whole input,
-//    12 bytes of DRAM traffic per value. The default for the scan from 2^18 values up to
+//    12 bytes of DRAM traffic per value. The default for the scan from 2^19 values up to
 //    the streamed pass below (4.25 TB/s at 2^28, where the streamed pass reaches 5.0), and
 //    for unaligned inputs. Below 2^22 the input stays in L2 between the kernels and what
 //    counts is the chain of look-backs, which the two kernels do not have. Microseconds,
 //    single pass (with its memset) / two kernels: scan 7.8/10.4 at 2^17, 8.4/8.2 at 2^18,
 //    10.1/8.2 at 2^19, 12.3/8.2 at 2^20, 15.2/10.3 at 2^21, equal at 2^22; compaction
-//    8.3/8.4, 10.2/8.2, 11.2/8.2, 15.3/10.3 and 17.3/10.4 at 2^17..2^21. The line is
-//    therefore 2^18 (kTwoPassFrom). An output that overlaps the input other than exactly
+//    8.3/8.4, 10.2/8.2, 11.2/8.2, 15.3/10.3 and 17.3/10.4 at 2^17..2^21. A call alone pays
+//    for the launch more: scan 10.6/12.4 at 2^18, 12.0/12.4 at 3 2^17, 12.2/12.4 at 2^19,
+//    15.5/12.5 at 2^20; compaction 12.5/12.6, 13.5/12.8, 14.7/12.7 and 17.0/13.7. The lines
+//    are therefore 2^19 and 2^18 (kTwoPassScan, kTwoPassCompact). An output that overlaps the input other than exactly
 //    in place keeps the single pass there, in which a tile writes only after all tiles
 //    before it have been read.
 //  - Wave form: one cooperative launch walks the input in waves of 2^24 values (64 MB,
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(kScanBlock, 6)
 //    re-read saves. Launch-shape variants 11-13 run the scan in waves of 2^22, 2^23 and
 //    2^24 values.
 constexpr int kChunkCtasPerSm = 4;
-constexpr long long kTwoPassFrom = 1LL << 18;  // two kernels by default
+constexpr long long kTwoPassScan = 1LL << 19, kTwoPassCompact = 1LL << 18;  // two kernels by default
 constexpr long long kTwoPassMinN = 1LL << 22;  // whatever the overlap; the wave variants
 constexpr long long kWaveValues = 1LL << 24;  // 64 MB of int32 per wave
 constexpr long long kWaveMinN = 1LL << 24;    // compaction: the wave form from here on
@@ -1030,7 +1032,7 @@ extern "C" hhs_status hhs_scan_exclusive_i32(const int32_t* d_in, int32_t* d_out
                                                          workspace_bytes, nullptr, nullptr, s);
         if (st != kStreamUnavailable) return st;
     }
-    const bool two_kernels = variant == 0 && n >= kTwoPassFrom &&
+    const bool two_kernels = variant == 0 && n >= kTwoPassScan &&
                              (d_in == d_out || !overlap(d_in, d_out, n));
     if (two_kernels ||
         ((variant == 0 || (variant >= 11 && variant <= 13)) && n >= kTwoPassMinN)) {
@@ -1101,7 +1103,7 @@ extern "C" hhs_status hhs_compact_flags_i32(const int32_t* d_flags, int32_t* d_s
     // an index list over the flags is filled behind the reads by the single pass only
     const bool apart = !overlap(d_flags, d_idx, n) &&
                        (!d_scan || d_scan == d_flags || !overlap(d_flags, d_scan, n));
-    if (n >= kTwoPassMinN || (n >= kTwoPassFrom && apart)) {
+    if (n >= kTwoPassMinN || (n >= kTwoPassCompact && apart)) {
         auto* agg = reinterpret_cast<unsigned*>(status);
         const size_t words =
             (scan_workspace_bytes(n, kScanMinTile) - sizeof(ScanHeader)) / sizeof(unsigned);

@@ -63,3 +63,17 @@ def test_compaction_forms(cuda, hhs, n, idx_over_flags, scan_out):
     assert np.array_equal(idx.cpu().numpy()[:len(ref)], ref)
     if scan is not None:
         assert np.array_equal(scan.cpu().numpy(), _exclusive(f))
+
+
+@pytest.mark.parametrize("n,kernels", [(EDGE, 1), (EDGE + 1, 1), (3 << 17, 1), (1 << 19, 2)])
+def test_scan_takes_a_second_kernel_where_it_pays(cuda, hhs, n, kernels):
+    """Below 2^19 values a single call takes longer with two kernels (12.4 us against 10.6). The single
+    pass clears the whole workspace, the two kernels write their chunk sums only."""
+    torch = cuda
+    a = torch.ones(n, dtype=torch.int32, device="cuda")
+    out = torch.empty_like(a)
+    ws, size = _ws(torch, hhs, n)
+    hhs.scan_exclusive_i32(_ptr(a), _ptr(out), n, _ptr(ws), size, None)
+    assert bool((ws == 0x5a).any()) == (kernels == 2)
+    assert hhs.scan_workspace_status(_ptr(ws), None) == 0
+    assert torch.equal(out, torch.arange(n, dtype=torch.int32, device="cuda"))
