@@ -1123,9 +1123,11 @@ __device__ void pack_ts(const EParams& E, const int32_t* S, int n, const Workers
 // tiles: so it is in systems with one dominating mass (the bounds hold m_i + m_max) and in units
 // that leave the range of the test's FP32 numbers. Milliseconds of timesteps a step, lists / without
 // the filter at all / with this choice: light disk around one mass, 16384 members 1.3 / 0.42 / 0.41,
-// 65536 102.7 / 8.0 / 7.8; 16384 in SI units 68 / 4.2 / 4.1. Elsewhere 0.2% to 0.5% pass.
+// 65536 102.7 / 8.0 / 7.8; 16384 in SI units 68 / 4.2 / 4.1. Elsewhere 0.2% to 0.5% pass. (Deciding
+// for nodes of 1024 members and more only: 12000 in SI units 5.4 / 2.5 / 2.5, two clusters far apart
+// 1.19 / 0.62 / 0.62 at 6001.)
 // FP64 keeps its lists (an FP64 evaluation of every pair takes longer than the lists do).
-constexpr int kTfDenseFrom = 1024;  // members; smaller nodes' pairs take a few microseconds anyway
+constexpr int kTfDenseFrom = 512;   // members (twice the sample)
 constexpr int kTfDensePass = 50;    // of 2048
 __device__ __forceinline__ bool tf_dense(const EParams& E, const int32_t* S, int n) {
     Smem& sm = cta_smem();
@@ -4640,7 +4642,7 @@ hhs_status engine_hold_step(hhs_ctx* c, const SoA& P, int n, double dt, bool cal
                               ? (pi == 0 ? subtree_launch(eh, k_subtree<HHS_PREC_FP64>, E, stream)
                                          : subtree_launch(eh, k_subtree<HHS_PREC_MIXED>, E, stream))
                           : pi == 0 ? engine_launch(eh, 0, k_engine<HHS_PREC_FP64, true>, E, stream)
-                          : n < kFilterN
+                          : n < kFilterN || !E.filter
                               ? engine_launch(eh, 1, k_engine<HHS_PREC_MIXED, false>, E, stream)
                               : engine_launch(eh, 1, k_engine<HHS_PREC_MIXED, true>, E, stream);
     hhs_count_launch();

@@ -210,3 +210,12 @@ def test_rows_whose_bound_was_too_high_fp64(cuda, hhs, oracle, n):
     out = d.download()
     for k in ("x", "y", "z", "vx", "vy", "vz", "ts"):
         assert np.array_equal(out[k], s[k]), k
+
+
+def test_step_in_other_units_small_nodes(cuda, hhs):
+    """A step whose nodes are mostly below 1024 members: 1.5 times the filtered phase (3.3 times when
+    those went through lists)."""
+    n = 12000
+    plain = _phases(hhs, hhs.plummer(n, 5), 1.0 / 64, 0.03, hhs.PREC_MIXED)["timesteps"]
+    s, dt = _units(hhs, n)
+    assert _phases(hhs, s, dt, 0.03, hhs.PREC_MIXED)["timesteps"] < 2.4 * plain
