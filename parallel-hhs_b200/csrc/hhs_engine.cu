@@ -4284,8 +4284,13 @@ std::array<const void*, 5> engine_kernels() {
 }
 // Mixed steps filter their timesteps from here on: at 16384 particles the filter saves 1.9 of 4.1
 // ms of timesteps, at 4099 0.04 of 0.41, and its code costs the subtree solver in the same kernel
-// 3% (registers). FP64 steps always do (a full FP64 evaluation takes ten times as long).
-constexpr int kFilterN = 6000;
+// 4 to 8% (registers; a function of its own costs the filter 10%). Milliseconds a step without /
+// with it, three mass spectra: 4099 3.1 to 3.5 / 3.3 to 3.6, 6001 5.0 to 5.4 / 5.2 to 5.6, 8192 6.9 to
+// 7.3 / 6.9 to 7.3, 9500 9.2 / 9.1, 12000 10.1 / 9.7, 16384 15.3 / 14.0, 20000 20.4 / 17.9; with a
+// quarter of the step 9500 2.34 / 2.36, 11000 2.34 / 2.31. A cold collapse, nearly all subtrees, loses
+// by it at any size: 16384 27.9 / 30.4. FP64 steps always filter (a full FP64 evaluation takes ten
+// times as long).
+constexpr int kFilterN = 10000;
 
 // The bound of a rate over the last one. In one timestep a rate changes by a factor of about
 // 1 +- 2 eta at most (it is |dv| / (eta r) or larger), so the guess has to fall with eta: a row
