@@ -128,9 +128,10 @@ typedef struct {
     int32_t warp_n;          /* nodes with at most warp_n (<= 32) particles run on one warp */
     int32_t cluster_size;    /* launch the persistent kernel in thread-block clusters (1,2,4,8,
                                 or 16 where the device allows clusters beyond 8) */
-    int32_t mid_n;           /* nodes with n <= mid_n (at most 640) run, with their whole subtree,
-                                from shared memory on the first cluster (on CTA 0 when
-                                cluster_size is 1); 0 = never */
+    int32_t mid_n;           /* nodes with n <= mid_n (at most 640; in FP64 steps at most 96: larger
+                                ones are faster on the grid) run, with their whole subtree, from
+                                shared memory on the first cluster (on CTA 0 when cluster_size
+                                is 1); 0 = never */
     int32_t packed;          /* mixed kick: two sinks per thread in packed FP32x2 arithmetic */
     int32_t mid_dist_n;      /* in such a subtree, nodes with more than mid_dist_n particles spread
                                 their pair work over the cluster's CTAs */
