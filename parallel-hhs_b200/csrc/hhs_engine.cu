@@ -3620,6 +3620,13 @@ __device__ __forceinline__ void mid_hold(const EParams& E, const int32_t* S, int
     mid_mark(E, sm, tm, 61);
 }
 
+// The FP64 solver for the device step's single-CTA subtrees, which only a caller's tuning sends there:
+// a second inlined copy would have the grid's one call its parts (8% of a step of 1024 particles).
+__device__ __noinline__ void mid_hold_fp64(const EParams& E, const int32_t* S, int n, int level0,
+                                           bool calc0, int dist_n, int cs, int rank) {
+    mid_hold<HHS_PREC_FP64>(E, S, n, level0, calc0, dist_n, cs, rank);
+}
+
 // FP64 rows as a function of the batched kernel, which has them in two places: inlined, its other
 // phases spill, and a function that took EParams by reference would put the system's copy of them
 // into local memory (as one for mid_hold did: 400 systems of up to 640 particles 9.3 ms, 8.5 with
@@ -3649,7 +3656,8 @@ __device__ __forceinline__ int mid_limit(const EParams& E) {
 // Walks the HOLD recursion from `top` (whose subsystem is already defined by the
 // counts/lists above it). Grid and cluster modes delegate nodes with n <= small_n,
 // with their whole subtree, to worker 0 alone.
-template <int PREC, int MODE, bool FILTER>
+// BATCH: in the batched kernel.
+template <int PREC, int MODE, bool FILTER, bool BATCH>
 __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers& W, Smem& sm,
                          unsigned long long& t_last) {
     unsigned long long after1 = 0, after2 = 0, calcm = 0;  // per-level state bits
@@ -3687,7 +3695,10 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                                        1, W.id - cs, W.count - cs, sm);
                     }
                 } else {
-                    mid_hold<PREC, true>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id, W.parts);
+                    if constexpr (PREC == HHS_PREC_FP64 && !BATCH)
+                        mid_hold_fp64(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id);
+                    else
+                        mid_hold<PREC, true>(E, S, n, lvl, calc, E.mid_dist_n, W.count, W.id, W.parts);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfCluster, 0.0, sm, lvl);
@@ -3707,7 +3718,7 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 if (W.id == 0) {
                     const Workers one{0, 1, kModeBlock};
                     unsigned long long t_sub = 0;
-                    run_hold<PREC, kModeBlock, false>(E, lvl, calc, one, sm, t_sub);
+                    run_hold<PREC, kModeBlock, false, BATCH>(E, lvl, calc, one, sm, t_sub);
                 }
                 if (!phase_barrier(E, sm, W)) return false;
                 prof_mark(E, W, t_last, kProfSubtree, 0.0, sm, lvl);
@@ -3773,7 +3784,8 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                     while (T > 8 && (n + T - 1) / T < W.count) T >>= 1;
                     for (int i0 = W.id * T; i0 < n; i0 += W.count * T) {
                         const int nrow = min(T, n - i0);
-                        ts_rows_fp64(E.P, S, n, i0, nrow, A);
+                        if constexpr (BATCH) ts_rows_fp64(E.P, S, n, i0, nrow, A);
+                        else ts_rows<PREC>(E.P, S, n, i0, nrow, A, sm.u.tr);
                         if ((int)threadIdx.x < nrow)
                             E.P.ts[list_at(S, i0 + threadIdx.x)] =
                                 ts_of_key<PREC>(sm.u.tr.best[threadIdx.x]);
@@ -3909,7 +3921,7 @@ __global__ void __launch_bounds__(kEB, 2) k_engine(const __grid_constant__ EPara
     unsigned long long t_last = 0;
     prof_begin(E, sm);
     prof_mark(E, W, t_last, -1, 0.0, sm);
-    run_hold<PREC, kModeGrid, FILTER>(E, E.top_level, E.calc_top != 0, W, sm, t_last);
+    run_hold<PREC, kModeGrid, FILTER, false>(E, E.top_level, E.calc_top != 0, W, sm, t_last);
     prof_end(E, sm);
 }
 
@@ -4222,7 +4234,7 @@ __global__ void __launch_bounds__(kEB, 2) k_batched(const __grid_constant__ BPar
         const int sys = B.order[idx];
         const EParams E = system_params(B, sys, B.cluster_slots + (size_t)cid * B.cluster_slot_bytes);
         const Workers W{rank, cs, kModeCluster, E.n_top > B.parts_n ? kBatchParts : 1};
-        run_hold<PREC, kModeCluster, false>(E, 0, E.calc_top != 0, W, sm, t);
+        run_hold<PREC, kModeCluster, false, true>(E, 0, E.calc_top != 0, W, sm, t);
     }
     // small systems: one CTA per system
     while (true) {
@@ -4234,7 +4246,7 @@ __global__ void __launch_bounds__(kEB, 2) k_batched(const __grid_constant__ BPar
         const int sys = B.order[B.n_big + idx];
         const EParams E = system_params(B, sys, B.cta_slots + (size_t)blockIdx.x * B.cta_slot_bytes);
         const Workers W{0, 1, kModeBlock};
-        run_hold<PREC, kModeBlock, false>(E, 0, E.calc_top != 0, W, sm, t);
+        run_hold<PREC, kModeBlock, false, true>(E, 0, E.calc_top != 0, W, sm, t);
     }
 }
 
