@@ -3714,17 +3714,21 @@ __device__ bool run_hold(const EParams& E, int top, bool top_calc, const Workers
                 lvl--;
                 continue;
             }
-            if (MODE != kModeBlock && n <= E.small_n) {
-                if (W.id == 0) {
-                    const Workers one{0, 1, kModeBlock};
-                    unsigned long long t_sub = 0;
-                    run_hold<PREC, kModeBlock, false, BATCH>(E, lvl, calc, one, sm, t_sub);
+            // (the mixed kernel with the filter is for tunings whose small_n the subtree solver covers:
+            // its code is 5% faster there without a second copy of the recursion)
+            if constexpr (MODE != kModeBlock && (!FILTER || PREC == HHS_PREC_FP64)) {
+                if (n <= E.small_n) {
+                    if (W.id == 0) {
+                        const Workers one{0, 1, kModeBlock};
+                        unsigned long long t_sub = 0;
+                        run_hold<PREC, kModeBlock, false, BATCH>(E, lvl, calc, one, sm, t_sub);
+                    }
+                    if (!phase_barrier(E, sm, W)) return false;
+                    prof_mark(E, W, t_last, kProfSubtree, 0.0, sm, lvl);
+                    calcm &= ~bit; after1 &= ~bit; after2 &= ~bit;
+                    lvl--;
+                    continue;
                 }
-                if (!phase_barrier(E, sm, W)) return false;
-                prof_mark(E, W, t_last, kProfSubtree, 0.0, sm, lvl);
-                calcm &= ~bit; after1 &= ~bit; after2 &= ~bit;
-                lvl--;
-                continue;
             }
             int nch = 1;
             bool filtered = false;
@@ -4296,11 +4300,11 @@ std::array<const void*, 5> engine_kernels() {
 }
 // Mixed steps filter their timesteps from here on: at 16384 particles the filter saves 1.9 of 4.1
 // ms of timesteps, at 4099 0.04 of 0.41, and its code costs the subtree solver in the same kernel
-// 4 to 8% (registers; a function of its own costs the filter 10%). Milliseconds a step without /
+// 3 to 5% (registers; a function of its own costs the filter 10%). Milliseconds a step without /
 // with it, three mass spectra: 4099 3.1 to 3.5 / 3.3 to 3.6, 6001 5.0 to 5.4 / 5.2 to 5.6, 8192 6.9 to
 // 7.3 / 6.9 to 7.3, 9500 9.2 / 9.1, 12000 10.1 / 9.7, 16384 15.3 / 14.0, 20000 20.4 / 17.9; with a
 // quarter of the step 9500 2.34 / 2.36, 11000 2.34 / 2.31. A cold collapse, nearly all subtrees, loses
-// by it at any size: 16384 27.9 / 30.4. FP64 steps always filter (a full FP64 evaluation takes ten
+// by it at any size: 16384 27.9 / 29.0. FP64 steps always filter (a full FP64 evaluation takes ten
 // times as long).
 constexpr int kFilterN = 10000;
 
@@ -4653,8 +4657,8 @@ hhs_status engine_hold_step(hhs_ctx* c, const SoA& P, int n, double dt, bool cal
     EParams E = engine_params(c, eh, P, n, dt, calc_ts, profile, top_level);
     const int pi = prec == HHS_PREC_FP64 ? 0 : 1;
     E.prec_mixed = pi;
-    if (pi == 1 && E.eta > kFilterEta) E.filter = 0;
     const int mid_n = std::min(pi == 0 ? std::min(eh->mid_n, kMidFp64) : eh->mid_n, kMid);
+    if (pi == 1 && (E.eta > kFilterEta || eh->small_n > mid_n)) E.filter = 0;
     const cudaError_t e = top_level == 0 && n <= mid_n
                               ? (pi == 0 ? subtree_launch(eh, k_subtree<HHS_PREC_FP64>, E, stream)
                                          : subtree_launch(eh, k_subtree<HHS_PREC_MIXED>, E, stream))

@@ -68,3 +68,24 @@ def test_collapse_below_the_line(cuda, hhs):
             now = ctx.profile()["cluster_node"]["ms"]
             best[calc], before = min(best[calc], now - before), now
     assert best[1] < 1.02 * best[0]
+
+
+@pytest.mark.parametrize("small_n,mid_n", [(64, 0), (700, 640), (128, 100), (640, 640)])
+def test_tunings_with_single_cta_nodes(cuda, hhs, small_n, mid_n):
+    """Nodes that the tuning gives to one CTA, above the subtree solver's size: steps without the
+    filter, which has no code for them. The same bits as from equal timesteps."""
+    n = 10007
+    s = hhs.plummer(n, 5)
+    a, b = hhs.ParticleSystem(n), hhs.ParticleSystem(n)
+    ctx = hhs.Context(n, 64, 0.03)
+    ctx.set_tuning(small_n=small_n, mid_n=mid_n)
+    a.upload(s)
+    b.upload(s)
+    hhs.hold_step(ctx, a, n, 0.0, 1.0 / 64, True, hhs.PREC_MIXED)
+    ctx.check()
+    hhs.timesteps(ctx, b, n, hhs.PREC_MIXED)
+    hhs.hold_step(ctx, b, n, 0.0, 1.0 / 64, False, hhs.PREC_MIXED)
+    ctx.check()
+    x, y = a.download(), b.download()
+    for k in ("x", "y", "z", "vx", "vy", "vz", "ts"):
+        assert np.array_equal(x[k], y[k]), k
