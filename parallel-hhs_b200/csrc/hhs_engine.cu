@@ -4800,7 +4800,7 @@ struct hhs_batch {
     hhs_params params{0.03, 0.0};
     int big_n[2] = {kMid, 1024};  // FP64, mixed: larger systems (n_big of them) get a cluster
     int n_big[2] = {0, 0}, n_clusters[2] = {0, 0};
-    int cluster_size = 8, small_n = 64, units_per_cta = 8, warp_n = 32, packed = 0;
+    int cluster_size[2] = {8, 8}, small_n = 64, units_per_cta = 8, warp_n = 32, packed = 0;
     int mid_n = kMid, mid_dist_n = 96;
     int parts_n = kBatchPartsN;  // big_n of mixed steps, once the caller or the tuner has set it
     void* arena = nullptr;
@@ -4857,40 +4857,46 @@ cudaError_t batched_occupancy(int cs, int* clusters) {
 // 60 2.5 / 4.2 and 4.0 / 4.4; where they are more than there are clusters of 4, 100 3.1 / 4.8 and with
 // 400 smaller ones 4.2 / 4.3, 170 4.7 / 4.7 and 5.7 / 4.8. So above that number only batches of at
 // most twice as many systems in all get them.
-bool batched_clusters(int cs, int* c0, int* c1) {
-    if (batched_occupancy<HHS_PREC_FP64>(cs, c0) == cudaSuccess &&
-        batched_occupancy<HHS_PREC_MIXED>(cs, c1) == cudaSuccess && *c0 > 0 && *c1 > 0)
+bool batched_clusters(int pi, int cs, int* n) {
+    if ((pi == 0 ? batched_occupancy<HHS_PREC_FP64>(cs, n)
+                 : batched_occupancy<HHS_PREC_MIXED>(cs, n)) == cudaSuccess && *n > 0)
         return true;
     (void)cudaGetLastError();
     return false;
 }
 
-bool batched_shape(hhs_batch* b, int* c0, int* c1) {
+bool batched_shape(hhs_batch* b) {
     // FP64 systems that one CTA does not hold in shared memory get a cluster (400 systems of 64 to
     // 2048: 34.5 ms, with 1024 as in mixed 41.5)
     int& big_n = b->big_n[1];
     big_n = b->n_max_sys > 1024 ? 1024 : kMid;
-    int large = 0, want = 4;
+    int large = 0, n = 0, want[2] = {4, 4};
     double e = 0.0;
-    for (const int n : b->sizes)
-        if (n > big_n) {
-            e += std::pow((double)n / b->n_max_sys, 2.33);
+    for (const int sz : b->sizes)
+        if (sz > big_n) {
+            e += std::pow((double)sz / b->n_max_sys, 2.33);
             large++;
         }
     if (b->n_max_sys > 1024) {
-        want = e < 8.0 ? 16 : (e < 40.0 ? 8 : 4);
+        want[0] = want[1] = e < 8.0 ? 16 : (e < 40.0 ? 8 : 4);
     } else {
         for (const int cs : {4, 8, 16}) {
-            if (!batched_clusters(cs, c0, c1)) continue;
-            if (large <= *c1) want = cs;
-            if (cs == 4 && large > *c1 && b->n_sys > 2 * *c1) big_n = 1024;
+            if (!batched_clusters(1, cs, &n)) continue;
+            if (large <= n) want[0] = want[1] = cs;
+            if (cs == 4 && large > n && b->n_sys > 2 * n) {
+                big_n = 1024;
+                want[1] = 8;  // 500 systems of 64 to 1024: 3.6 ms with a CTA each, 4.3 in a
+                break;        // launch of clusters of 4; FP64, in clusters, 16.9 and 13.3
+            }
         }
     }
-    for (const int cs : {want, 8}) {  // the portable size is the fallback
-        b->cluster_size = cs;
-        if (batched_clusters(cs, c0, c1)) return true;
+    for (int pi = 0; pi < 2; pi++) {
+        b->cluster_size[pi] = want[pi];
+        if (batched_clusters(pi, want[pi], &b->n_clusters[pi])) continue;
+        b->cluster_size[pi] = 8;  // the portable size is the fallback
+        if (!batched_clusters(pi, 8, &b->n_clusters[pi])) return false;
     }
-    return false;
+    return true;
 }
 
 void batch_set_big(hhs_batch* b, int pi, int big_n) {
@@ -4933,15 +4939,12 @@ extern "C" hhs_status hhs_batch_create(int32_t n_sys, const int32_t* offsets, in
     std::iota(b->order.begin(), b->order.end(), 0);
     std::stable_sort(b->order.begin(), b->order.end(),
                      [&](int a, int c) { return b->sizes[a] > b->sizes[c]; });
-    int c0 = 0, c1 = 0;
-    if (!batched_shape(b, &c0, &c1)) {
+    if (!batched_shape(b)) {
         delete b;
         return HHS_ERR_CUDA;
     }
-    b->n_clusters[0] = c0;
-    b->n_clusters[1] = c1;
-    b->max_clusters = c0 > c1 ? c0 : c1;
-    b->max_ctas = b->max_clusters * b->cluster_size;
+    b->max_clusters = std::max(b->n_clusters[0], b->n_clusters[1]);
+    b->max_ctas = std::max(b->n_clusters[0] * b->cluster_size[0], b->n_clusters[1] * b->cluster_size[1]);
     size_t offc[5], offs[5];
     b->cluster_slot_bytes = slot_layout(b->n_max_sys, b->max_levels, kMaxChunks, offc);
     b->cta_slot_bytes = slot_layout(b->n_max_sys, b->max_levels, 1, offs);
@@ -5072,13 +5075,13 @@ extern "C" hhs_status hhs_hold_batched(hhs_batch* b, hhs_particle_system* sys, d
     B.off_k = b->off_k; B.off_tiles = b->off_tiles; B.off_rate = b->off_rate;
     B.leaf_times = b->d_leaf;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nclu * b->cluster_size, 1, 1);
+    cfg.gridDim = dim3(nclu * b->cluster_size[pi], 1, 1);
     cfg.blockDim = dim3(kEB, 1, 1);
     cfg.dynamicSmemBytes = kEngineSmem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = b->cluster_size;
+    at[0].val.clusterDim.x = b->cluster_size[pi];
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
