@@ -824,7 +824,8 @@ __device__ void ts_sym_tiles(const EParams& E, int n, int cw, long long u0, long
 // CTA's), since the reduction itself changes the velocities.
 // Measured: the timestep phases of an N=65536 step (Salpeter masses) 123.0 -> 41 ms, 16384 4.10 ->
 // 2.24 (FP64: 40.7 -> 2.6); a calc of 64678 members 1.21 ms, 1.7e12 unordered pairs/s. What
-// bounds it: the FMA pipe (half busy) and, below about 6000 members, the latency of the tiles.
+// bounds it, by count: ten FMA lanes a pair are 46% of the pipe in large nodes; below about 6000
+// members the latency of the tiles.
 constexpr float kTfAlpha = 0.8f;
 constexpr float kTfAll = 1.0e38f;   // a particle whose pairs all pass
 
@@ -3931,8 +3932,8 @@ __global__ void __launch_bounds__(kEB, 2) k_engine(const __grid_constant__ EPara
 
 // A system that the subtree solver takes whole: one cluster instead of a cooperative launch of the
 // whole GPU with its barrier and look-back words cleared first, and a kernel without the grid
-// phases' registers (256 particles: 319 -> 290 us). What bounds it is the solver's latency: over a
-// hundred nodes one after another, most of them on one warp.
+// phases' registers (256 particles: within the spread of runs to 9% less). What bounds it is the
+// solver's latency: over a hundred nodes one after another, most of them on one warp.
 template <int PREC>
 __global__ void __launch_bounds__(kEB, 1) k_subtree(const __grid_constant__ EParams E) {
     Smem& sm = cta_smem();
