@@ -936,7 +936,7 @@ __device__ __forceinline__ void tf_merge(const EParams& E, const int32_t* S, int
     if constexpr (PREC == HHS_PREC_FP64) {
         const double t = tf_tau(E, gi, gj);
         if (t < 1.e30) {
-            const unsigned long long key = ~(unsigned long long)__double_as_longlong(t);
+            const unsigned long long key = ~(unsigned long long)__double_as_longlong(f64_add(t, 0.0));
             atomicMax(&E.tau_key[i], key);
             atomicMax(&E.tau_key[j], key);
         }

@@ -76,7 +76,8 @@ __device__ __forceinline__ unsigned long long ts_key(const TsState& a, const TsS
         double t = kHuge;
         ts_pair_fp64(f64_sub(a.x, b.x), f64_sub(a.y, b.y), f64_sub(a.z, b.z), f64_sub(a.vx, b.vx),
                      f64_sub(a.vy, b.vy), f64_sub(a.vz, b.vz), a.m, b.m, A.eta, A.eta_s2, t);
-        return t < kHuge ? ~(unsigned long long)__double_as_longlong(t) : 0ull;
+        // (+ 0: a coincident pair of negative mass sum has a timescale of -0, the least there is)
+        return t < kHuge ? ~(unsigned long long)__double_as_longlong(f64_add(t, 0.0)) : 0ull;
     } else {
         const DS ax = ds_split(a.x), ay = ds_split(a.y), az = ds_split(a.z);
         const DS bx = ds_split(b.x), by = ds_split(b.y), bz = ds_split(b.z);

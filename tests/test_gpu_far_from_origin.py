@@ -43,3 +43,20 @@ def test_kick_sf_mixed_odd_slices(cuda, hhs, oracle, n_sink, n_src):
     acc = oracle.kick(sink, src, 1.0)
     # the bound of a mixed pair term, and what the positions lose
     assert np.all(np.abs(dv - acc) <= 5e-7 * mag + LOST * slope)
+
+
+@pytest.mark.parametrize("n", [20, 100, 2500])
+def test_fp64_timestep_of_a_coincident_pair_of_negative_mass(cuda, hhs, oracle, n):
+    """Its timescale is -0, below every other, and every calculation of the pair gives it."""
+    s = hhs.plummer(n, 5)
+    for k in ("x", "y", "z"):
+        s[k][3] = s[k][n - 2]
+    s["m"][3] = -2.0 * s["m"][n - 2]
+    ref = oracle.timesteps(s, 0.03)
+    assert ref[3] == 0.0 and ref[n - 2] == 0.0
+    d = hhs.ParticleSystem(n)
+    d.upload(s)
+    hhs.timesteps(hhs.Context(n, 8, 0.03), d, n, hhs.PREC_FP64)
+    got = d.download()["ts"]
+    assert got[3] == 0.0 and got[n - 2] == 0.0
+    assert np.array_equal(got, ref)
